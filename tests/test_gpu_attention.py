@@ -440,3 +440,73 @@ def test_decode_shapes_kv_longer_or_shorter_than_q(cuda, Sq, Sk):
     Sk > Sq, down to a single query row), GQA heads, no mask."""
     q, k, v = _qkv(2, Sq, Sk, 8, 2, 128, seed=Sq * 7 + Sk)
     _check(cuda, q, k, v)
+
+
+@pytest.mark.parametrize("Sq,Sk,Hq,Hk,D,causal,window,alibi", [
+    (1, 1, 8, 2, 128, False, None, False),        # one key: three warps of the CTA have none
+    (1, 15, 4, 4, 64, False, None, True),         # less than one 16-key tile, one row per tile
+    (1, 17, 32, 1, 128, False, None, False),      # MQA: 32 packed rows, two row tiles
+    (3, 63, 8, 2, 64, True, None, True),          # rows that see one to three keys
+    (5, 65, 12, 4, 128, False, None, False),      # 15 of 16 packed rows live
+    (16, 4093, 8, 2, 128, False, (1 << 29, 4077), False),  # causal, aligned at the end of the cache
+    (16, 300, 8, 1, 64, False, (1 << 29, 284), False),     # 128 packed rows: four double row tiles
+    (2, 2100, 8, 8, 128, False, (100, 2098), False),       # a left edge inside the keys
+    (9, 700, 6, 2, 128, False, (3, 2), True),     # a window of a few keys: most splits are empty
+    (16, 5, 4, 2, 64, False, (2, 1), False),      # rows beyond the keys: nothing visible, output 0
+    (17, 300, 8, 2, 128, False, None, False),     # one row more than the decode kernel takes
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_query_rows(cuda, Sq, Sk, Hq, Hk, D, causal, window, alibi, dtype):
+    """Few query rows against many keys: packed row tiles, key splits and their merge, at the edges
+    of the 16-key tiles, the 16-row tiles and the splits. Bound: probabilities are rounded to
+    2^-9 (bf16) of themselves and so is the result, each at most 2^-9 * max|v| ~ 9e-3."""
+    q, k, v = _qkv(3, Sq, Sk, Hq, Hk, D, seed=Sq * 31 + Sk, dtype=dtype)
+    slopes = R.alibi_slopes_ref(Hq) if alibi else None
+    from trinix_b200 import ops
+    out, lse = ops.attention(q.to(cuda), k.to(cuda), v.to(cuda), causal=causal, window=window,
+                             alibi_slopes=None if slopes is None else slopes.to(cuda),
+                             return_lse=True)
+    assert T.attention_status(cuda) == 0
+    qf, kf, vf = q.float(), k.float(), v.float()
+    ref = R.attention_variant_ref(qf, kf, vf, None, causal, window, slopes)
+    s = torch.einsum("bihd,bjhd->bhij", qf, R.tile_kv_heads_ref(kf, Hq // Hk)) * D ** -0.5
+    i, j = torch.arange(Sq)[:, None], torch.arange(Sk)[None]
+    if slopes is not None:
+        s = s - slopes.view(1, -1, 1, 1) * (i - j).abs()
+    if causal:
+        s = s.masked_fill(j > i, float("-inf"))
+    if window is not None:
+        s = s.masked_fill((j - i < -window[0]) | (j - i > window[1]), float("-inf"))
+    ref_lse = torch.logsumexp(s, -1)
+    seen = ~torch.isinf(ref_lse)
+    assert torch.equal(torch.isinf(lse.cpu()), ~seen)
+    # fp32 scores of 128 terms of magnitude ~1 and fp32 sums: 1e-5 each
+    assert float((lse.cpu()[seen] - ref_lse[seen]).abs().max()) <= 5e-5
+    rows = seen.transpose(1, 2)
+    assert float((out.float().cpu()[rows] - ref[rows]).abs().max()) <= TOL
+    assert not out.float().cpu()[~rows].any()
+
+
+@pytest.mark.parametrize("Sq", [1, 4])
+def test_few_query_rows_in_every_layout(cuda, Sq):
+    """The same call with contiguous tensors, transposed (B, H, S, D) storage, a slice of a longer
+    cache, expanded kv heads (of both tensors and of K alone) and an expanded batch."""
+    q, k, v = _qkv(2, Sq, 333, 8, 2, 128, seed=Sq)
+    q, k, v = q.to(cuda), k.to(cuda), v.to(cuda)
+    base = T.triton_attn_func(q, k, v)
+    swap = lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)  # noqa: E731
+    assert torch.equal(T.triton_attn_func(swap(q), swap(k), swap(v)), base)
+    cache = torch.full((2, 512, 2, 128), float("nan"), device=cuda, dtype=k.dtype)
+    cache[:, 40:373] = k  # the keys around the slice are never used
+    assert torch.equal(T.triton_attn_func(q, cache[:, 40:373], v), base)
+    k1, v1 = k[:, :, :1], v[:, :, :1]
+    mqa = T.triton_attn_func(q, k1, v1)
+    assert torch.equal(T.triton_attn_func(q, k1.expand(-1, -1, 8, -1), v1.expand(-1, -1, 8, -1)), mqa)
+    half = T.triton_attn_func(q, k1.expand(-1, -1, 2, -1), v)  # K shared by all heads, V by four
+    ref = R.attention_variant_ref(q.float().cpu(), k1.expand(-1, -1, 2, -1).float().cpu(),
+                                  v.float().cpu())
+    assert float((half.float().cpu() - ref).abs().max()) <= TOL
+    kb, vb = k[:1].expand(2, -1, -1, -1), v[:1].expand(2, -1, -1, -1)
+    assert torch.equal(T.triton_attn_func(q, kb, vb),
+                       T.triton_attn_func(q, kb.contiguous(), vb.contiguous()))
+    assert T.attention_status(cuda) == 0

@@ -21,6 +21,7 @@
 // h / (Hq / Hk), so GQA / MQA need no tiled copies. With ALiBi under a causal mask the KV tiles
 // of a row block are visited from the diagonal backwards: the bias grows with the key index, so
 // in that order the first tile holds the row maximum and O is never rescaled again.
+// Calls of up to 16 query rows without mask or dropout take the kernel of attention_decode.cuh.
 //
 // Every wait on an mbarrier is bounded: after a fixed number of polls the kernel records a
 // code in the status word of the caller's workspace, raises a CTA-wide abort flag, drains its
@@ -63,6 +64,10 @@ struct AttnParams {
   int B, Sq, Sk, Hq;
   int k_hdiv, v_hdiv;  // query heads per kv head (Hq when the tensor's heads are collapsed)
   int k_bmul, v_bmul;  // 1, or 0 when the batch dim is broadcast
+  int group;           // consecutive query heads that read one kv head in K and in V
+  int decode;          // few query rows: attention_decode.cuh
+  const void* q;       // read directly by the decode kernel
+  long long q_stride_b, q_stride_s, q_stride_h;
   long long o_stride_b, o_stride_s, o_stride_h;
   long long lse_stride_b, lse_stride_h;
   float scale_log2;    // softmax scale * log2(e)
@@ -1058,10 +1063,10 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// (D, S, H, B) view of a (B, S, H, D) tensor with element strides (b, s, h); box = 64 x 128.
+// (D, S, H, B) view of a (B, S, H, D) tensor with element strides (b, s, h); box = 64 x box_rows.
 // Dims with stride 0 (broadcast) are collapsed to size 1 by the caller.
 static int make_map(CUtensorMap* tm, const void* base, int is_bf16, int64_t D, int64_t S,
-                    int64_t H, int64_t B, int64_t sb, int64_t ss, int64_t sh) {
+                    int64_t H, int64_t B, int64_t sb, int64_t ss, int64_t sh, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return TRX_ERR_CUDA;
   if (!aligned_to(base, 16)) return TRX_ERR_ALIGNMENT;
@@ -1077,7 +1082,7 @@ static int make_map(CUtensorMap* tm, const void* base, int is_bf16, int64_t D, i
                            static_cast<cuuint64_t>(sb * 2)};
   for (int i = 0; i < 3; ++i)
     if (strides[i] >= (1ull << 40)) return TRX_ERR_STRIDE;
-  cuuint32_t box[4] = {64, static_cast<cuuint32_t>(ATT_BM), 1, 1};
+  cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(tm, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                    4, const_cast<void*>(base), dims, strides, box, estr,
@@ -1115,6 +1120,8 @@ static int launch_attn(const AttnParams& p, cudaStream_t stream) {
 }
 
 }  // namespace trx
+
+#include "attention_decode.cuh"
 
 using namespace trx;
 
@@ -1165,7 +1172,8 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
 
   p = AttnParams{};
   const int is_bf16 = dtype == TRX_BF16;
-  int rc = make_map(&p.tm_q, q, is_bf16, D, Sq, Hq, B, q_strides[0], q_strides[1], q_strides[2]);
+  int rc = make_map(&p.tm_q, q, is_bf16, D, Sq, Hq, B, q_strides[0], q_strides[1], q_strides[2],
+                    ATT_BM);
   if (rc != TRX_OK) return rc;
   // Broadcast (stride-0) head or batch dims of k / v collapse to extent 1.
   const int64_t Sk_map = Sk > 0 ? Sk : 1;
@@ -1173,11 +1181,17 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   const void* vv = Sk > 0 ? v : q;
   const bool k_hb = (Hk > 1 && k_strides[2] == 0), v_hb = (Hk > 1 && v_strides[2] == 0);
   const bool k_bb = (B > 1 && k_strides[0] == 0), v_bb = (B > 1 && v_strides[0] == 0);
+  const int group = static_cast<int>(Hq / Hk);
+  p.k_hdiv = k_hb ? static_cast<int>(Hq) : group;
+  p.v_hdiv = v_hb ? static_cast<int>(Hq) : group;
+  p.group = p.k_hdiv < p.v_hdiv ? p.k_hdiv : p.v_hdiv;
+  p.decode = !bias && dropout_p == 0.0f && use_decode(Sq, Hq, p.group) ? 1 : 0;
+  const int kv_box = p.decode ? DEC_KEYS : ATT_BN;
   rc = make_map(&p.tm_k, kk, is_bf16, D, Sk_map, k_hb ? 1 : Hk, k_bb ? 1 : B, k_strides[0],
-                k_strides[1], k_strides[2]);
+                k_strides[1], k_strides[2], kv_box);
   if (rc != TRX_OK) return rc;
   rc = make_map(&p.tm_v, vv, is_bf16, D, Sk_map, v_hb ? 1 : Hk, v_bb ? 1 : B, v_strides[0],
-                v_strides[1], v_strides[2]);
+                v_strides[1], v_strides[2], kv_box);
   if (rc != TRX_OK) return rc;
   p.out = out;
   p.lse = lse_or_null;
@@ -1187,9 +1201,10 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   p.Sq = static_cast<int>(Sq);
   p.Sk = static_cast<int>(Sk);
   p.Hq = static_cast<int>(Hq);
-  const int group = static_cast<int>(Hq / Hk);
-  p.k_hdiv = k_hb ? static_cast<int>(Hq) : group;
-  p.v_hdiv = v_hb ? static_cast<int>(Hq) : group;
+  p.q = q;
+  p.q_stride_b = q_strides[0];
+  p.q_stride_s = q_strides[1];
+  p.q_stride_h = q_strides[2];
   p.k_bmul = k_bb ? 0 : 1;
   p.v_bmul = v_bb ? 0 : 1;
   p.o_stride_b = o_strides[0];
@@ -1232,6 +1247,14 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
 
 static int attn_fwd_launch(const AttnParams& p, int64_t D, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (p.decode) {
+    const bool wide = p.group * p.Sq > 16;
+    if (D == 128)
+      return p.is_bf16 ? (wide ? launch_decode<128, true, 2>(p, s) : launch_decode<128, true, 1>(p, s))
+                       : (wide ? launch_decode<128, false, 2>(p, s) : launch_decode<128, false, 1>(p, s));
+    return p.is_bf16 ? (wide ? launch_decode<64, true, 2>(p, s) : launch_decode<64, true, 1>(p, s))
+                     : (wide ? launch_decode<64, false, 2>(p, s) : launch_decode<64, false, 1>(p, s));
+  }
   if (D == 128) return p.is_bf16 ? launch_attn<128, true>(p, s) : launch_attn<128, false>(p, s);
   return p.is_bf16 ? launch_attn<64, true>(p, s) : launch_attn<64, false>(p, s);
 }
