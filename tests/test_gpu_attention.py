@@ -510,3 +510,30 @@ def test_few_query_rows_in_every_layout(cuda, Sq):
     assert torch.equal(T.triton_attn_func(q, kb, vb),
                        T.triton_attn_func(q, kb.contiguous(), vb.contiguous()))
     assert T.attention_status(cuda) == 0
+
+
+@pytest.mark.parametrize("Sk", [1, 31, 33, 127, 258, 264, 509])
+@pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (64, torch.float16)])
+@pytest.mark.parametrize("wide", [True, False])
+def test_dense_mask_at_every_alignment(cuda, Sk, D, dtype, wide):
+    """The mask in fp32 and in the activation dtype, with rows that allow copies of 16, 4 and 2
+    bytes (row lengths that are multiples of 8, even, odd; a view one element into its storage),
+    keys hidden by -inf and by the type's lowest value, ragged last tiles. Bound as for the other
+    masks: probabilities and result are each rounded once, 2^-9 * max|v| in bf16."""
+    B, Sq, H = 2, 150, 4
+    q, k, v = _qkv(B, Sq, Sk, H, 2, D, seed=Sk, dtype=dtype)
+    mdt = torch.float32 if wide else dtype
+    g = torch.Generator().manual_seed(Sk + D)
+    mask = torch.randn(B, 1, Sq, Sk, generator=g)
+    mask[torch.rand(B, 1, Sq, Sk, generator=g) < 0.2] = float("-inf")
+    mask[:, :, :, 0] = 0.0  # every row sees a key
+    if Sk > 8:
+        mask[1, :, :, 5] = torch.finfo(mdt).min
+    mask = mask.to(mdt)
+    store = torch.zeros(mask.numel() + 1, dtype=mdt, device=cuda)
+    for shift in (0, 1):
+        m = store[shift:shift + mask.numel()].view(mask.shape).copy_(mask.to(cuda))
+        out = T.triton_attn_func(q.to(cuda), k.to(cuda), v.to(cuda), attn_mask=m)
+        assert T.attention_status(cuda) == 0
+        _, ref32 = _mask_ref(q, k, v, mask.float(), False)
+        assert float((out.float().cpu() - ref32).abs().max()) <= TOL

@@ -82,6 +82,7 @@ struct AttnParams {
   const void* bias;
   long long bias_sb, bias_sh, bias_sq;  // elements
   int bias_kind;       // 0 none, 1 fp32, 2 the activation dtype
+  int bias_copy;       // bytes of one copy that every row's alignment allows: 16, 4 or 2
   // dropout on the normalised probabilities: an element is dropped when its random byte is
   // below drop_thr (0 = no dropout); kept ones are scaled by drop_scale = 256 / (256 - drop_thr)
   unsigned drop_thr;
@@ -329,18 +330,29 @@ __host__ __device__ constexpr uint32_t make_idesc(int is_bf16, int m, int n, int
          (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-template <int D>
+// What an instantiation carries: nothing beyond causal / window / ALiBi; dropout; a dense additive
+// mask with or without dropout.
+enum AttnFeature { ATT_PLAIN = 0, ATT_DROPOUT = 1, ATT_MASK_F32 = 2, ATT_MASK_16 = 3 };
+__host__ __device__ constexpr bool feature_has_mask(int f) { return f >= ATT_MASK_F32; }
+
+// With a mask each softmax warp has MASK_BUFS buffers of 16 rows x 32 mask values; at head dim 128
+// they take the room of two K/V tiles (the softmax on a masked tile is longer than a tile's load).
+template <int D, int FEATURE>
 struct AttnSmem {
+  static constexpr int STAGES = feature_has_mask(FEATURE) && D > 64 ? 2 : ATT_STAGES;
+  static constexpr int MASK_BUFS = feature_has_mask(FEATURE) ? 2 : 0;
+  static constexpr int MASK_CHUNK = 16 * 128;
   static constexpr int CHUNKS = D / 64;              // 64-element (128-byte) column chunks
   static constexpr int CHUNK_BYTES = ATT_BN * 128;   // 128 rows x 128 B = 16 KB
   static constexpr int TILE_BYTES = CHUNKS * CHUNK_BYTES;
   static constexpr int Q_OFF = 0;
   static constexpr int KV_OFF = ATT_NQ * TILE_BYTES;
-  static constexpr int BAR_OFF = KV_OFF + ATT_STAGES * TILE_BYTES;
-  static constexpr int NUM_BARS = 2 + 2 * ATT_STAGES + 6 + 1 + 2;
+  static constexpr int BAR_OFF = KV_OFF + STAGES * TILE_BYTES;
+  static constexpr int NUM_BARS = 2 + 2 * STAGES + 6 + 1 + 2;
   static constexpr int XCH_OFF = BAR_OFF + NUM_BARS * 8 + 64;      // row max / sum exchange
   static constexpr int XCH_BYTES = ATT_NQ * 2 * ATT_BM * 4;
-  static constexpr int TOTAL = XCH_OFF + XCH_BYTES;
+  static constexpr int MASK_OFF = (XCH_OFF + XCH_BYTES + 127) / 128 * 128;
+  static constexpr int TOTAL = MASK_OFF + ATT_SM_WARPS * MASK_BUFS * MASK_CHUNK;
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for 1024-byte alignment
 };
 
@@ -363,12 +375,11 @@ __device__ __forceinline__ TileRange tile_range(const AttnParams& p, int row0) {
   return r;
 }
 
-// BIAS: the instantiation with the rarely used features — a dense additive mask and / or dropout,
-// each behind a run-time flag; the other instantiation carries none of it.
-template <int D, bool BF16, bool BIAS>
+template <int D, bool BF16, int FEATURE>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
     attn_fwd_kernel(const __grid_constant__ AttnParams p) {
-  using L = AttnSmem<D>;
+  using L = AttnSmem<D, FEATURE>;
+  constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -378,8 +389,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   // barrier indices
   constexpr int B_QFULL = 0;                        // [2]
   constexpr int B_KVFULL = 2;                       // [STAGES]
-  constexpr int B_KVEMPTY = 2 + ATT_STAGES;         // [STAGES]
-  constexpr int B_SFULL = 2 + 2 * ATT_STAGES;       // [2]
+  constexpr int B_KVEMPTY = 2 + STAGES;         // [STAGES]
+  constexpr int B_SFULL = 2 + 2 * STAGES;       // [2]
   constexpr int B_PFULL = B_SFULL + 2;              // [2]
   constexpr int B_ODONE = B_PFULL + 2;              // [2]
   constexpr int B_DRAIN = B_ODONE + 2;              // [1]
@@ -422,11 +433,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   const int kv_first = p.reverse_kv ? JHI - 1 : JLO;
   // One K or V tile into ring stage fill % STAGES (K and V tiles alternate: even fills are K).
   auto issue_fill = [&](int fill) {
-    const int s = fill % ATT_STAGES;
+    const int s = fill % STAGES;
     const int j = kv_first + (fill >> 1) * kv_step;
     const bool is_k = (fill & 1) == 0;
     mbar_expect_tx(bar(B_KVFULL + s), L::TILE_BYTES);
-    fills_issued[s] = fill / ATT_STAGES + 1;
+    fills_issued[s] = fill / STAGES + 1;
     const CUtensorMap* tm = is_k ? &p.tm_k : &p.tm_v;
     const int hh = h / (is_k ? p.k_hdiv : p.v_hdiv);
     const int bb = b * (is_k ? p.k_bmul : p.v_bmul);
@@ -443,7 +454,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   if (warp == ATT_SM_WARPS && lane == 0 && !skip_launch) {
     mbar_init(bar(B_QFULL + 0), 1);
     mbar_init(bar(B_QFULL + 1), 1);
-    for (int s = 0; s < ATT_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(bar(B_KVFULL + s), 1);
       mbar_init(bar(B_KVEMPTY + s), 1);
       fills_issued[s] = 0;
@@ -473,7 +484,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         }
       }
       // the ring is empty: its first round of fills waits for nobody
-      const int first_round = min(ATT_STAGES, 2 * (JHI - JLO));
+      const int first_round = min(STAGES, 2 * (JHI - JLO));
       for (int fill = 0; fill < first_round; ++fill) issue_fill(fill);
     }
   }
@@ -502,9 +513,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       // Q and the first round of the ring were issued before the CTA-wide sync
       const int total = 2 * (JHI - JLO);
       bool ok = true;
-      for (int fill = ATT_STAGES; fill < total && ok; ++fill) {
-        const uint32_t par = ((fill / ATT_STAGES) & 1) ^ 1;
-        ok = mbar_wait(bar(B_KVEMPTY + fill % ATT_STAGES), par, abort_flag, p.status,
+      for (int fill = STAGES; fill < total && ok; ++fill) {
+        const uint32_t par = ((fill / STAGES) & 1) ^ 1;
+        ok = mbar_wait(bar(B_KVEMPTY + fill % STAGES), par, abort_flag, p.status,
                        ATT_ST_PRODUCER);
         if (ok) issue_fill(fill);
       }
@@ -514,7 +525,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     if (lane == 0 && JHI > JLO) {
       const uint32_t idesc_qk = make_idesc(BF16 ? 1 : 0, ATT_BM, ATT_BN, 0, 0);
       const uint32_t idesc_pv = make_idesc(BF16 ? 1 : 0, ATT_BM, D, 0, 1);
-      static_assert((ATT_STAGES & (ATT_STAGES - 1)) == 0, "ring depth must be a power of two");
+      static_assert((STAGES & (STAGES - 1)) == 0, "ring depth must be a power of two");
       // This thread sits between the softmax warps and the tensor pipe: every cycle it spends
       // between two groups of MMAs is a cycle the pipe idles once its short queue has drained
       // (the same 32 MMAs per KV tile issued from a loop with per-tile state in arrays, lambdas
@@ -592,9 +603,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         const int jp = rev ? JHI - 1 - r : JLO + r;  // KV tile of the P V
         const int jq = rev ? jp - 1 : jp + 1;        // KV tile of the next Q K^T
         const uint32_t fv = static_cast<uint32_t>(f + 1), fk = static_cast<uint32_t>(f + 2);
-        const uint32_t sv = fv & (ATT_STAGES - 1), sk = fk & (ATT_STAGES - 1);
-        if (has_pv) ok = wait(B_KVFULL + sv, (fv / ATT_STAGES) & 1);
-        if (ok && has_qk) ok = wait(B_KVFULL + sk, (fk / ATT_STAGES) & 1);
+        const uint32_t sv = fv & (STAGES - 1), sk = fk & (STAGES - 1);
+        if (has_pv) ok = wait(B_KVFULL + sv, (fv / STAGES) & 1);
+        if (ok && has_qk) ok = wait(B_KVFULL + sk, (fk / STAGES) & 1);
         const uint32_t vst = v_lo + sv * T16, kst = k_lo + sk * T16;
         if (ok && (STEADY || (has_pv && jp >= jlo0 && jp < jhi0))) {
           ok = wait(B_PFULL + 0, ppar0);
@@ -696,24 +707,71 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const float sl2 = p.scale_log2;
     const float slope2 = p.slopes ? p.slopes[hq] * 1.4426950408889634f : 0.0f;
     const bool has_alibi = p.slopes != nullptr;
-    const bool has_bias = BIAS && p.bias_kind != 0;
-    const bool has_drop = BIAS && p.drop_thr != 0u;
-    // rows of the dense mask that this thread's two score rows read (valid rows only)
-    const uint8_t* brow[2] = {nullptr, nullptr};
-    if (has_bias) {
-      const int esz = p.bias_kind == 1 ? 4 : 2;
+    constexpr bool has_bias = feature_has_mask(FEATURE);
+    const bool has_drop = FEATURE != ATT_PLAIN && p.drop_thr != 0u;
+    // The mask values of this warp's 16 rows come into shared memory by cp.async, 32 columns (one
+    // chunk of 16 rows x 128 bytes) at a time and MASK_BUFS chunks ahead of their use: a copy of the
+    // warp covers whole row segments (one or two cache lines each, any alignment), and its latency
+    // runs under the work on the chunks before. Read straight from global memory in the layout of
+    // the scores, a request touches eight rows and its latency lies on the softmax chain. Kernel
+    // times, fp32 mask, 8 x 16 heads, head dim 64, 509 x 509 (4-byte copies) / 512 x 512 (16-byte):
+    // 206 / 132 us read where used, 69 / 64 us with the loads batched in front of the wait for the
+    // scores, 64 / 46 us this way (29 us without a mask). 4 x 16 heads x 2048^2, head dim 128:
+    // 997 -> 291 us.
+    // Chunk layout: row r at 128 r; its 8-column group g at 32 (g ^ (r & 3)), fp32 or 16-bit values.
+    const uint32_t mask_ring = sbase + L::MASK_OFF + warp * (L::MASK_BUFS * L::MASK_CHUNK);
+    const int mask_row0 = row0 + wq * 32 + sub * 16;
+    constexpr int ESZ = FEATURE == ATT_MASK_F32 ? 4 : 2;
+    auto copy_rows = [&](auto bytes_tag, int n, int tile) {
+      constexpr int BYTES = decltype(bytes_tag)::value;     // of one copy
+      constexpr int PER = BYTES / ESZ, LANES = 32 / PER;    // values of a copy, copies of a row
+      constexpr int STEP = 32 / LANES;                      // rows of one pass of the warp
+      const int c = lane % LANES * PER, r0 = lane / LANES;
+      const int col = tile * ATT_BN + (n & 3) * 32 + c;
+      const int live = max(0, min(PER, p.Sk - col)) * ESZ;  // the rest is filled with zeros
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.bias) +
+                           ESZ * (b * p.bias_sb + hq * p.bias_sh + (mask_row0 + r0) * p.bias_sq +
+                                  (live > 0 ? col : 0));
+      const uint32_t dst = mask_ring + (n % L::MASK_BUFS) * L::MASK_CHUNK + r0 * 128 +
+                           (((c >> 3) ^ (r0 & 3)) << 5) + (c & 7) * ESZ;
+      const int rows = p.Sq - mask_row0 - r0;  // of the mask from this lane's first one on
 #pragma unroll
-      for (int hr = 0; hr < 2; ++hr)
-        if (row0 + rl + 8 * hr < p.Sq)
-          brow[hr] = reinterpret_cast<const uint8_t*>(p.bias) +
-                     esz * (b * p.bias_sb + hq * p.bias_sh +
-                            static_cast<long long>(row0 + rl + 8 * hr) * p.bias_sq);
-    }
+      for (int k = 0; k < 16; k += STEP) {
+        const uint32_t to = (dst ^ ((k & 3) << 5)) + k * 128;
+        const int size = k < rows ? live : 0;
+        if constexpr (BYTES == 16)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(size)
+                       : "memory");
+        else if constexpr (BYTES == 4)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(size)
+                       : "memory");
+        else
+          asm volatile("st.shared.u16 [%0], %1;" ::"r"(to),
+                       "h"(size ? __ldg(reinterpret_cast<const unsigned short*>(src))
+                                : static_cast<unsigned short>(0))
+                       : "memory");
+        if (k + STEP < 16 && k + STEP < rows) src += ESZ * STEP * p.bias_sq;
+      }
+    };
+    auto copy_mask = [&](int n, int tile) {  // chunk n of this warp: columns 32 (n % 4) of KV tile
+      if (p.bias_copy == 16) copy_rows(std::integral_constant<int, 16>{}, n, tile);
+      else if (p.bias_copy == 4) copy_rows(std::integral_constant<int, 4>{}, n, tile);
+      else if constexpr (ESZ == 2) copy_rows(std::integral_constant<int, 2>{}, n, tile);
+    };
+    auto mask_commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
     const int j_first = p.reverse_kv ? rng[t].jhi - 1 : rng[t].jlo;  // first KV tile visited
     float m_run[2] = {-INFINITY, -INFINITY};  // reference max (log2 domain) per row
     float l_run[2] = {0.0f, 0.0f};            // this thread's share of the row sums
     bool ok = true;
+    if constexpr (has_bias) {
+      if (n_it > 0)
+#pragma unroll 1
+        for (int n = 0; n < L::MASK_BUFS; ++n) {
+          copy_mask(n, j_first);
+          mask_commit();
+        }
+    }
 
     for (int itn = 0; itn < n_it && ok; ++itn) {
       const int j = j_first + itn * kv_step;
@@ -738,10 +796,80 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         else if (c0 >= row1) alibi_sgn = -1;          // every key at or after every query
       }
       // general path: a tile that straddles the diagonal under ALiBi, or a non-positive scale
-      const bool general = (has_alibi && alibi_sgn == 0) || !(sl2 > 0.0f) || has_bias || has_drop;
+      const bool general = (has_alibi && alibi_sgn == 0) || !(sl2 > 0.0f) || has_drop;
       float m_tile[2] = {-INFINITY, -INFINITY};
       float off[2] = {0.0f, 0.0f};  // fast path: x = t * sl2 + off
-      if (general) {
+      auto max_of_tile = [&](float unit) {  // of scores that become x = t * unit + off
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+          float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+          for (int g = 0; g < 16; g += 2) {
+            mx0 = max3(mx0, __uint_as_float(sr[4 * g + 2 * hr]), __uint_as_float(sr[4 * g + 2 * hr + 1]));
+            mx1 = max3(mx1, __uint_as_float(sr[4 * g + 4 + 2 * hr]),
+                       __uint_as_float(sr[4 * g + 5 + 2 * hr]));
+          }
+          const float mraw = fmaxf(mx0, mx1);
+          m_tile[hr] = (mraw == -INFINITY) ? -INFINITY : fmaf(mraw, unit, off[hr]);
+        }
+      };
+      if constexpr (has_bias) {
+        // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf
+        const float2 scale2 = make_float2(sl2, sl2);
+        const float2 log2e2 = make_float2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(L::MASK_BUFS - 1) : "memory");
+          __syncwarp();
+          const int n = 4 * itn + c;
+          const uint32_t from = mask_ring + (c % L::MASK_BUFS) * L::MASK_CHUNK + (lane >> 2) * 128;
+#pragma unroll
+          for (int g = 4 * c; g < 4 * c + 4; ++g) {
+            const uint32_t at = from + (((g & 3) ^ ((lane >> 2) & 3)) << 5);
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+              float2 bv;
+              if constexpr (FEATURE == ATT_MASK_F32) {
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                             : "=f"(bv.x), "=f"(bv.y)
+                             : "r"(at + hr * 1024 + q4 * 8)
+                             : "memory");
+              } else {
+                uint32_t u;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"(at + hr * 1024 + q4 * 4)
+                             : "memory");
+                bv = Pack<std::conditional_t<BF16, __nv_bfloat16, __half>>::cvt2(u);
+              }
+              const int i = 4 * g + 2 * hr;
+              float2 x = mul2(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), scale2);
+              if (has_alibi) {
+                const float d = static_cast<float>(row_g[hr] - c0 - 8 * g - 2 * q4);
+                x.x = fmaf(-slope2, fabsf(d), x.x);
+                x.y = fmaf(-slope2, fabsf(d - 1.0f), x.y);
+              }
+              x = fma2(bv, log2e2, x);
+              sr[i] = __float_as_uint(x.x);
+              sr[i + 1] = __float_as_uint(x.y);
+            }
+          }
+          __syncwarp();  // every lane has read the chunk
+          const int next = n + L::MASK_BUFS;
+          if (next < 4 * n_it) copy_mask(next, j_first + (next >> 2) * kv_step);
+          mask_commit();
+        }
+        if (need_mask) {
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {
+            const int lo_c = lo_i[hr] - c0 - 2 * q4, hi_c = hi_i[hr] - c0 - 2 * q4;
+#pragma unroll
+            for (int g = 0; g < 16; ++g)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                if (8 * g + e < lo_c || 8 * g + e > hi_c) sr[4 * g + 2 * hr + e] = 0xff800000u;
+          }
+        }
+        max_of_tile(1.0f);
+      } else if (general) {
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
           const float fi = static_cast<float>(row_g[hr] - c0 - 2 * q4);
@@ -752,16 +880,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
               const int i = 4 * g + 2 * hr + e;
               float x = __uint_as_float(sr[i]) * sl2;
               if (has_alibi) x = fmaf(-slope2, fabsf(fi - static_cast<float>(8 * g + e)), x);
-              if (has_bias) {
-                const int col = c0 + 8 * g + 2 * q4 + e;
-                if (brow[hr] != nullptr && col < p.Sk) {
-                  float bv;
-                  if (p.bias_kind == 1) bv = reinterpret_cast<const float*>(brow[hr])[col];
-                  else if (BF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(brow[hr])[col]);
-                  else bv = __half2float(reinterpret_cast<const __half*>(brow[hr])[col]);
-                  x = fmaf(bv, 1.4426950408889634f, x);  // -inf stays -inf
-                }
-              }
               if (need_mask) {
                 const int col = c0 + 8 * g + 2 * q4 + e;
                 if (col < lo_i[hr] || col > hi_i[hr]) x = -INFINITY;
@@ -826,18 +944,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             cp = add2(cp, step);
           }
         }
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-          for (int g = 0; g < 16; g += 2) {
-            mx0 = max3(mx0, __uint_as_float(sr[4 * g + 2 * hr]), __uint_as_float(sr[4 * g + 2 * hr + 1]));
-            mx1 = max3(mx1, __uint_as_float(sr[4 * g + 4 + 2 * hr]),
-                       __uint_as_float(sr[4 * g + 5 + 2 * hr]));
-          }
-          const float mraw = fmaxf(mx0, mx1);
-          m_tile[hr] = (mraw == -INFINITY) ? -INFINITY : fmaf(mraw, sl2, off[hr]);
-        }
+        max_of_tile(sl2);
       }
       // the four threads of a quad hold the four column slices of the same two rows
 #pragma unroll
@@ -865,7 +972,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       // P = exp2(x - m_ref), packed to 16-bit pairs IN PLACE: sr[2g + hr] = P(row hr, column
       // 4g + q4). Slot 2g + hr never lies ahead of the scores still to be read (4g + 2hr ..).
       float2 lsum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-      if (general) {
+      if (has_bias ? has_drop : general) {
         uint4 rnd[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
 #pragma unroll
         for (int g = 0; g < 16; ++g) {
@@ -895,7 +1002,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
           }
         }
       } else {
-        const float2 sc2 = make_float2(sl2, sl2);
+        const float unit = has_bias ? 1.0f : sl2;  // a mask's scores are scaled already
+        const float2 sc2 = make_float2(unit, unit);
         const float2 nm2[2] = {make_float2(off[0] - m_ref[0], off[0] - m_ref[0]),
                                make_float2(off[1] - m_ref[1], off[1] - m_ref[1])};
 #pragma unroll
@@ -936,6 +1044,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       if (lane == 0) mbar_arrive(bar(B_PFULL + t));
     }
 
+    if constexpr (has_bias) asm volatile("cp.async.wait_all;" ::: "memory");
     // ---- epilogue: O / l -> global --------------------------------------------------
     // Row statistics go through shared memory once: xch[0][row] = row sum, xch[1][row] = max.
     if (ok) {
@@ -967,7 +1076,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       const float l_row = xch[r];
       const float m_row = xch[ATT_BM + r];
       float inv = (n_it > 0 && l_row > 0.0f) ? __fdividef(1.0f, l_row) : 0.0f;
-      if (BIAS && p.drop_thr != 0u) inv *= p.drop_scale;  // kept probabilities count 1 / (1 - p)
+      if (FEATURE != ATT_PLAIN && p.drop_thr != 0u) inv *= p.drop_scale;  // kept probabilities count 1 / (1 - p)
       const uint32_t o_addr = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + 2 * ATT_BN +
                               t * ATT_BN + sub * OC;
       uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) +
@@ -1012,7 +1121,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) {
     // make sure no bulk copy of this CTA is still in flight before shared memory is released
-    for (int s = 0; s < ATT_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       const int n = fills_issued[s];
       if (n > 0) {
         bool done = false;
@@ -1091,8 +1200,8 @@ static int make_map(CUtensorMap* tm, const void* base, int is_bf16, int64_t D, i
   return r == CUDA_SUCCESS ? TRX_OK : TRX_ERR_CUDA;
 }
 
-template <int D, bool BF16, bool BIAS>
-static int launch_attn_bias(const AttnParams& p, cudaStream_t stream) {
+template <int D, bool BF16, int FEATURE>
+static int launch_attn_feature(const AttnParams& p, cudaStream_t stream) {
   // The attribute is set once per device; host threads that race on the first call each set
   // the same value (the call is idempotent) and publish the flag atomically.
   static std::atomic<bool> configured[64];
@@ -1100,23 +1209,25 @@ static int launch_attn_bias(const AttnParams& p, cudaStream_t stream) {
   if (cudaGetDevice(&dev) != cudaSuccess) return TRX_ERR_CUDA;
   const bool cacheable = dev >= 0 && dev < 64;
   if (!cacheable || !configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<D, BF16, BIAS>,
+    if (cudaFuncSetAttribute(attn_fwd_kernel<D, BF16, FEATURE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             AttnSmem<D>::DYN_BYTES) != cudaSuccess)
+                             AttnSmem<D, FEATURE>::DYN_BYTES) != cudaSuccess)
       return TRX_ERR_CUDA;
     if (cacheable) configured[dev].store(true, std::memory_order_release);
   }
   const int rows_per_cta = p.pair_heads ? ATT_BM : ATT_NQ * ATT_BM;
   const int mblocks = (p.Sq + rows_per_cta - 1) / rows_per_cta;
   dim3 grid(mblocks, p.pair_heads ? p.Hq / 2 : p.Hq, p.B);
-  attn_fwd_kernel<D, BF16, BIAS><<<grid, ATT_THREADS, AttnSmem<D>::DYN_BYTES, stream>>>(p);
+  attn_fwd_kernel<D, BF16, FEATURE><<<grid, ATT_THREADS, AttnSmem<D, FEATURE>::DYN_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? TRX_OK : TRX_ERR_CUDA;
 }
 
 template <int D, bool BF16>
 static int launch_attn(const AttnParams& p, cudaStream_t stream) {
-  return (p.bias_kind != 0 || p.drop_thr != 0u) ? launch_attn_bias<D, BF16, true>(p, stream)
-                                                : launch_attn_bias<D, BF16, false>(p, stream);
+  if (p.bias_kind == 1) return launch_attn_feature<D, BF16, ATT_MASK_F32>(p, stream);
+  if (p.bias_kind == 2) return launch_attn_feature<D, BF16, ATT_MASK_16>(p, stream);
+  if (p.drop_thr != 0u) return launch_attn_feature<D, BF16, ATT_DROPOUT>(p, stream);
+  return launch_attn_feature<D, BF16, ATT_PLAIN>(p, stream);
 }
 
 }  // namespace trx
@@ -1231,6 +1342,12 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
     p.bias_sh = bias_strides[1];
     p.bias_sq = bias_strides[2];
     p.bias_kind = bias_dtype == TRX_F32 ? 1 : 2;
+    const int64_t esz = p.bias_kind == 1 ? 4 : 2;
+    auto copies_of = [&](int64_t bytes) {
+      return aligned_to(bias, bytes) && bias_strides[0] * esz % bytes == 0 &&
+             bias_strides[1] * esz % bytes == 0 && bias_strides[2] * esz % bytes == 0;
+    };
+    p.bias_copy = copies_of(16) ? 16 : copies_of(4) ? 4 : static_cast<int>(esz);
   }
   if (dropout_p > 0.0f) {
     // the drop probability is realised in steps of 1/256 (one random byte per element)
