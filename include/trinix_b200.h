@@ -274,6 +274,26 @@ int trx_residual_layernorm_bwd(const void* dy, const void* x, const void* residu
                                void* stream);
 
 /*
+ * Backward of (residual) RMSNorm / LayerNorm with the forward's row statistics instead of
+ * recomputed ones: rstd (and mean) are the fp32 [R] outputs of trx_rmsnorm_fwd,
+ * trx_residual_rmsnorm_fwd, trx_layernorm_fwd or trx_residual_layernorm_fwd on the same rows.
+ * res_or_null is the residual of the residual forms. Otherwise as trx_rmsnorm_bwd /
+ * trx_layernorm_bwd (same workspace, same results up to the statistics' last bits). Replaces nothing
+ * beyond what those two replace.
+ */
+int trx_rmsnorm_bwd_saved(const void* dy, const void* x, const void* res_or_null, const void* w,
+                          const float* rstd, void* dx, void* dw_or_null, int64_t R, int64_t C,
+                          int64_t dy_row_stride, int64_t x_row_stride, int64_t res_row_stride,
+                          int64_t dx_row_stride, int x_dtype, int w_dtype, void* workspace,
+                          size_t workspace_bytes, void* stream);
+int trx_layernorm_bwd_saved(const void* dy, const void* x, const void* res_or_null,
+                            const void* w_or_null, const float* mean, const float* rstd, void* dx,
+                            void* dw_or_null, void* db_or_null, int64_t R, int64_t C,
+                            int64_t dy_row_stride, int64_t x_row_stride, int64_t res_row_stride,
+                            int64_t dx_row_stride, int x_dtype, int wb_dtype, void* workspace,
+                            size_t workspace_bytes, void* stream);
+
+/*
  * Backward of act(RMSNorm(x)) (trx_rmsnorm_act_fwd): with z = w * n the upstream gradient becomes
  * dy * act'(z), then as trx_rmsnorm_bwd (same workspace). act is one of TRX_ACT_*.
  * Replaces TritonFusedRMSNormActivationFunction.backward

@@ -333,3 +333,37 @@ def test_empty_and_invalid_backward_inputs(cuda):
         T.ops.glu_backward(x, x, "swiglu")
     with pytest.raises(ValueError):
         T.ops.rmsnorm_backward(x.cpu(), x.cpu(), w.cpu(), 1e-6)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 1000), (64, 4096), (3, 4104), (2, 16384), (3, 777)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_norm_backward_with_the_forwards_statistics(cuda, rows, cols, dtype):
+    """The forward's rstd (and mean) against recomputed ones, in every width class and on the scalar
+    path, with and without a residual. The statistics differ in their last fp32 bits only (sums in
+    another order, 2^-22 relative), so the fp32 gradients differ by a few times that and 16-bit ones
+    by at most one rounding (2^-8 / 2^-11 of the value, twice half an ulp)."""
+    g = torch.Generator().manual_seed(rows + cols)
+    x, r, dy = (torch.randn(rows, cols, generator=g).to(dtype).to(cuda) for _ in range(3))
+    w, b = (torch.randn(cols, generator=g).to(dtype).to(cuda) for _ in range(2))
+    tol = {torch.float32: 5e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+
+    def close(a, b):  # relative to the value, or to the rms where the value is a small difference
+        a, b = a.double(), b.double()
+        return bool(((a - b).abs() <= tol * (b.abs() + b.pow(2).mean().sqrt())).all())
+
+    for res in (None, r):
+        if res is None:
+            _, rstd = T.ops.rmsnorm(x, w, 1e-6, return_rstd=True)
+            _, mean, ln_rstd = T.ops.layernorm(x, w, b, 1e-6, return_stats=True)
+        else:
+            _, rstd = T.ops.residual_rmsnorm(x, res, w, 1e-6, return_rstd=True)
+            _, mean, ln_rstd = T.ops.residual_layernorm(x, res, w, b, 1e-6, return_stats=True)
+        for saved, again in zip(T.ops.rmsnorm_backward(dy, x, w, 1e-6, residual=res, rstd=rstd),
+                                T.ops.rmsnorm_backward(dy, x, w, 1e-6, residual=res)):
+            assert close(saved, again)
+        for saved, again in zip(
+                T.ops.layernorm_backward(dy, x, w, 1e-6, residual=res, mean=mean, rstd=ln_rstd),
+                T.ops.layernorm_backward(dy, x, w, 1e-6, residual=res)):
+            assert close(saved, again)
+    with pytest.raises(ValueError):
+        T.ops.rmsnorm_backward(dy, x, w, 1e-6, rstd=torch.ones(rows + 1, device=cuda))

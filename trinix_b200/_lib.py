@@ -58,6 +58,13 @@ SIGNATURES = {
     "trx_layernorm_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_int64, c_int64, c_int64, c_int64, c_int64, c_float, c_int,
                                   c_int, c_void_p, c_size_t, c_void_p]),
+    "trx_rmsnorm_bwd_saved": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                      c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
+                                      c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "trx_layernorm_bwd_saved": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                        c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64,
+                                        c_int64, c_int64, c_int64, c_int, c_int, c_void_p, c_size_t,
+                                        c_void_p]),
     "trx_residual_rmsnorm_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
                                          c_float, c_int, c_int, c_void_p, c_size_t, c_void_p]),

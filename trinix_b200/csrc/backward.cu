@@ -2,8 +2,10 @@
 //
 // Norms. A CTA of 128 to 512 threads walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; a row of x and
 // of dy is read from HBM once with 128-bit streaming loads and stays in registers. The row's
-// statistics are recomputed from x (nothing has to be saved by the forward), dx is written, and
-// every thread keeps fp32 running sums of dy * n (and dy) for the columns it owns. At the end
+// statistics are the forward's (SAVED) or recomputed from x; what bounds the kernel is the latency
+// of the CTA-wide reductions of a row at 12 to 24 warps per SM, and the saved statistics leave one
+// of three (LayerNorm, 32768 x 4096 bf16: 166.4 -> 151.5 us) or of two (RMSNorm: 149.6 -> 136.4
+// us). dx is written, and every thread keeps fp32 running sums of dy * n (and dy) for the columns it owns. At the end
 // each CTA writes its sums as one row of a (P, C) fp32 block in the caller's workspace and a
 // second kernel adds the P rows in a fixed order: dW and db are deterministic for a given shape
 // and device. (The reference accumulates dW across programs under spin locks,
@@ -49,6 +51,8 @@ struct NormBwdParams {
   void* dx;
   float* dw_part;    // (P, C) fp32 or null
   float* db_part;    // (P, C) fp32 or null
+  const float* mean;  // (R) row statistics as the forward had them, or null: recomputed from x
+  const float* rstd;
   float* stats;      // (R, 2) fp32: mean, rstd (scalar path only)
   int64_t R, C;
   int64_t dy_stride, x_stride, dx_stride, res_stride;  // elements
@@ -118,8 +122,9 @@ __device__ __forceinline__ float act_grad(int act, float z) {
   return 2.0f * fmaxf(z, 0.0f);
 }
 
-template <bool LN, typename T, int VPT, int NT>
-__global__ void __launch_bounds__(NT, NT <= 256 ? (LN ? TRX_BWD_MINB_LN : TRX_BWD_MINB_RMS) : 1) norm_bwd_kernel(const NormBwdParams p) {
+template <bool LN, bool SAVED, typename T, int VPT, int NT>
+__global__ void __launch_bounds__(NT, NT <= 256 ? (LN ? TRX_BWD_MINB_LN : TRX_BWD_MINB_RMS) : 1)
+    norm_bwd_kernel(const NormBwdParams p) {
   using P = Pack<T>;
   constexpr int VEC = P::VEC;
   __shared__ float2 red[2][NT / 32];
@@ -142,6 +147,11 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? (LN ? TRX_BWD_MINB_LN : TRX_BW
   for (int64_t row = blockIdx.x; row < p.R; row += gridDim.x) {
     const T* xrow = reinterpret_cast<const T*>(p.x) + row * p.x_stride;
     const T* grow = reinterpret_cast<const T*>(p.dy) + row * p.dy_stride;
+    float mean = 0.0f, rstd = 0.0f;
+    if constexpr (SAVED) {
+      if constexpr (LN) mean = __ldg(p.mean + row);
+      rstd = __ldg(p.rstd + row);
+    }
     uint4 xr[VPT], gr[VPT];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -180,9 +190,16 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? (LN ? TRX_BWD_MINB_LN : TRX_BW
         }
       }
     }
-    // ---- statistics, recomputed from x --------------------------------------------
-    float mean = 0.0f, rstd;
-    if constexpr (LN) {
+    // ---- statistics: the forward's, or recomputed from x ----------------------------
+    if constexpr (SAVED) {
+      if constexpr (LN) {
+        const float2 nmean2 = make_float2(-mean, -mean);
+#pragma unroll
+        for (int i = 0; i < VPT; ++i)
+#pragma unroll
+          for (int j = 0; j < H2; ++j) xf[i][j] = add2(xf[i][j], nmean2);
+      }
+    } else if constexpr (LN) {
       float2 s2 = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
@@ -304,18 +321,21 @@ __global__ void __launch_bounds__(256) norm_bwd_generic_dx(const NormBwdParams p
       const float f = P::load1(xrow + c);
       return rrow ? f + P::load1(rrow + c) : f;
     };
-    float mean = 0.0f;
-    if constexpr (LN) {
+    float mean = LN && p.rstd ? p.mean[row] : 0.0f;
+    if (LN && !p.rstd) {
       float s = 0.0f;
       for (int64_t c = threadIdx.x; c < p.C; c += 256) s += xval(c);
       mean = block_sum2(make_float2(s, 0.0f), red, sel).x * inv_C;
     }
-    float cs = 0.0f;
-    for (int64_t c = threadIdx.x; c < p.C; c += 256) {
-      const float d = xval(c) - mean;
-      cs = fmaf(d, d, cs);
+    float rstd = p.rstd ? p.rstd[row] : 0.0f;
+    if (!p.rstd) {
+      float cs = 0.0f;
+      for (int64_t c = threadIdx.x; c < p.C; c += 256) {
+        const float d = xval(c) - mean;
+        cs = fmaf(d, d, cs);
+      }
+      rstd = rsqrtf(fmaf(block_sum2(make_float2(cs, 0.0f), red, sel).x, inv_C, p.eps));
     }
-    const float rstd = rsqrtf(fmaf(block_sum2(make_float2(cs, 0.0f), red, sel).x, inv_C, p.eps));
     float c1 = 0.0f, c2 = 0.0f;
     for (int64_t c = threadIdx.x; c < p.C; c += 256) {
       const float n = (xval(c) - mean) * rstd;
@@ -415,7 +435,7 @@ static int64_t norm_bwd_partial_rows(int64_t R, int64_t C) {
 
 // TRX_BWD_WAVES resident waves of CTAs (each walks R / grid rows); P_rows comes back as the grid size, i.e.
 // the number of rows of partial sums that were written.
-template <bool LN, typename T, int VPT, int NT>
+template <bool LN, bool SAVED, typename T, int VPT, int NT>
 static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStream_t stream) {
   static std::atomic<int> blocks_per_sm_of[64];  // racing first calls store the same value
   int dev = 0;
@@ -424,7 +444,7 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   int blocks_per_sm = cacheable ? blocks_per_sm_of[dev].load(std::memory_order_acquire) : 0;
   if (blocks_per_sm == 0) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, T, VPT, NT>, NT, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, SAVED, T, VPT, NT>, NT, 0) !=
             cudaSuccess || n <= 0)
       n = 1;
     blocks_per_sm = n;
@@ -432,7 +452,27 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   }
   const int64_t resident = static_cast<int64_t>(sm_count_of_current_device()) * blocks_per_sm * TRX_BWD_WAVES;
   if (P_rows > resident) P_rows = resident;
-  norm_bwd_kernel<LN, T, VPT, NT><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
+  norm_bwd_kernel<LN, SAVED, T, VPT, NT><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
+}
+
+template <bool LN, bool SAVED, typename T>
+static void launch_norm_bwd_width(const NormBwdParams& p, int64_t nvec, int64_t& P_rows,
+                                  cudaStream_t stream) {
+  // few vectors per thread: the running column sums cost 8 (16 for LayerNorm) registers each
+  if (nvec <= 256) {
+    launch_norm_bwd_vec<LN, SAVED, T, 1, 256>(p, P_rows, stream);
+  } else if (nvec <= 512) {
+    // measured on 32768 x 4096 bf16, statistics recomputed: RMSNorm 256 threads x 2 vectors (146
+    // us; 159 us at 128 x 4), LayerNorm 128 x 4 (170 us; 188 us at 256 x 2): LayerNorm then has
+    // three CTA-wide reductions per row, which four warps finish sooner than eight; 512 threads x
+    // 1 vector is slower for both (213 / 278 us). With the forward's statistics, one reduction:
+    // RMSNorm 136.4 us (156 / 234 us at 2 / 4 CTAs per SM), LayerNorm 151.5 us at 128 x 4 (163.5 us
+    // at 256 x 2; 175.6 / 218.8 us at 2 / 4 CTAs per SM)
+    constexpr int V = LN ? 4 : TRX_BWD512_VPT;
+    launch_norm_bwd_vec<LN, SAVED, T, V, 512 / V>(p, P_rows, stream);
+  } else {
+    launch_norm_bwd_vec<LN, SAVED, T, 2, 512>(p, P_rows, stream);
+  }
 }
 
 template <bool LN, typename T>
@@ -452,17 +492,8 @@ static int launch_norm_bwd(NormBwdParams p, void* dw, void* db, float* ws, cudaS
     if (p.res) vec_ok = vec_ok && aligned_to(p.res, 16) && (p.res_stride % VEC == 0);
     const int64_t nvec = p.C / VEC;
     if (vec_ok && nvec <= 1024) {
-      // few vectors per thread: the running column sums cost 8 (16 for LayerNorm) registers each
-      if (nvec <= 256) launch_norm_bwd_vec<LN, T, 1, 256>(p, P_rows, stream);
-      else if (nvec <= 512) {
-        // measured on 32768 x 4096 bf16: RMSNorm 256 threads x 2 vectors (146 us; 159 us at
-        // 128 x 4), LayerNorm 128 x 4 (170 us; 188 us at 256 x 2): LayerNorm has three CTA-wide
-        // reductions per row, which four warps finish sooner than eight; 512 threads x 1 vector
-        // is slower for both (213 / 278 us)
-        if constexpr (LN) launch_norm_bwd_vec<LN, T, 4, 128>(p, P_rows, stream);
-        else launch_norm_bwd_vec<LN, T, TRX_BWD512_VPT, 512 / TRX_BWD512_VPT>(p, P_rows, stream);
-      }
-      else launch_norm_bwd_vec<LN, T, 2, 512>(p, P_rows, stream);
+      if (p.rstd) launch_norm_bwd_width<LN, true, T>(p, nvec, P_rows, stream);
+      else launch_norm_bwd_width<LN, false, T>(p, nvec, P_rows, stream);
     } else {
       const int64_t cap = static_cast<int64_t>(sm_count_of_current_device()) * 8;
       norm_bwd_generic_dx<LN, T><<<static_cast<unsigned>(p.R < cap ? p.R : cap), 256, 0, stream>>>(p);
@@ -498,7 +529,8 @@ static int norm_bwd_entry(const void* dy, const void* x, const void* w, void* dx
                           int64_t R, int64_t C, int64_t dy_stride, int64_t x_stride,
                           int64_t dx_stride, float eps, int x_dtype, int w_dtype, void* workspace,
                           size_t workspace_bytes, void* stream, const void* res = nullptr,
-                          int64_t res_stride = 0, int act = -1) {
+                          int64_t res_stride = 0, int act = -1, const float* mean = nullptr,
+                          const float* rstd = nullptr) {
   if (!bwd_dtype_ok(x_dtype) || !bwd_dtype_ok(w_dtype)) return TRX_ERR_DTYPE;
   if (R < 0 || C <= 0) return TRX_ERR_SHAPE;
   if (R > 0 && (!dy || !x || !dx)) return TRX_ERR_NULL_POINTER;
@@ -511,7 +543,7 @@ static int norm_bwd_entry(const void* dy, const void* x, const void* w, void* dx
   NormBwdParams p{};
   p.dy = dy; p.x = x; p.w = w; p.dx = dx; p.res = res; p.res_stride = res_stride;
   p.R = R; p.C = C; p.dy_stride = dy_stride; p.x_stride = x_stride; p.dx_stride = dx_stride;
-  p.eps = eps; p.w_dtype = w_dtype; p.act = act;
+  p.eps = eps; p.w_dtype = w_dtype; p.act = act; p.mean = mean; p.rstd = rstd;
   float* ws = static_cast<float*>(workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (x_dtype) {
@@ -662,6 +694,31 @@ extern "C" int trx_layernorm_bwd(const void* dy, const void* x, const void* w_or
   return norm_bwd_entry<true>(dy, x, w_or_null, dx, dw_or_null, db_or_null, R, C, dy_row_stride,
                               x_row_stride, dx_row_stride, eps, x_dtype, wb_dtype, workspace,
                               workspace_bytes, stream);
+}
+
+extern "C" int trx_rmsnorm_bwd_saved(const void* dy, const void* x, const void* res_or_null,
+                                     const void* w, const float* rstd, void* dx, void* dw_or_null,
+                                     int64_t R, int64_t C, int64_t dy_row_stride,
+                                     int64_t x_row_stride, int64_t res_row_stride,
+                                     int64_t dx_row_stride, int x_dtype, int w_dtype,
+                                     void* workspace, size_t workspace_bytes, void* stream) {
+  if (R > 0 && !rstd) return TRX_ERR_NULL_POINTER;
+  return norm_bwd_entry<false>(dy, x, w, dx, dw_or_null, nullptr, R, C, dy_row_stride, x_row_stride,
+                               dx_row_stride, 0.0f, x_dtype, w_dtype, workspace, workspace_bytes,
+                               stream, res_or_null, res_row_stride, -1, nullptr, rstd);
+}
+
+extern "C" int trx_layernorm_bwd_saved(const void* dy, const void* x, const void* res_or_null,
+                                       const void* w_or_null, const float* mean, const float* rstd,
+                                       void* dx, void* dw_or_null, void* db_or_null, int64_t R,
+                                       int64_t C, int64_t dy_row_stride, int64_t x_row_stride,
+                                       int64_t res_row_stride, int64_t dx_row_stride, int x_dtype,
+                                       int wb_dtype, void* workspace, size_t workspace_bytes,
+                                       void* stream) {
+  if (R > 0 && (!mean || !rstd)) return TRX_ERR_NULL_POINTER;
+  return norm_bwd_entry<true>(dy, x, w_or_null, dx, dw_or_null, db_or_null, R, C, dy_row_stride,
+                              x_row_stride, dx_row_stride, 0.0f, x_dtype, wb_dtype, workspace,
+                              workspace_bytes, stream, res_or_null, res_row_stride, -1, mean, rstd);
 }
 
 extern "C" int trx_residual_rmsnorm_bwd(const void* dy, const void* x, const void* residual,

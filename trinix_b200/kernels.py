@@ -54,19 +54,20 @@ def _run(fn, *args):
 
 
 class _RMSNormFn(torch.autograd.Function):
-    """Counterpart of TritonRMSNormFunction (trinix/kernels/rmsnorm_kernel.py:197-321). Saves x and
-    w only: the backward kernel recomputes the row statistics."""
+    """Counterpart of TritonRMSNormFunction (trinix/kernels/rmsnorm_kernel.py:197-321). Saves x, w
+    and the fp32 row statistics, as the reference does."""
 
     @staticmethod
     def forward(ctx, X, W, eps):
-        ctx.save_for_backward(X, W)
+        y, rstd = ops.rmsnorm(X, W, eps, return_rstd=True)
+        ctx.save_for_backward(X, W, rstd)
         ctx.eps = eps
-        return ops.rmsnorm(X, W, eps)
+        return y
 
     @staticmethod
     def backward(ctx, dY):
-        X, W = ctx.saved_tensors
-        dx, dw = ops.rmsnorm_backward(dY, X, W, ctx.eps, need_dw=ctx.needs_input_grad[1])
+        X, W, rstd = ctx.saved_tensors
+        dx, dw = ops.rmsnorm_backward(dY, X, W, ctx.eps, need_dw=ctx.needs_input_grad[1], rstd=rstd)
         return dx, dw, None
 
 
@@ -75,17 +76,18 @@ class _LayerNormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, X, W, b, eps):
-        ctx.save_for_backward(X, W)
+        y, mean, rstd = ops.layernorm(X, W, b, eps, return_stats=True)
+        ctx.save_for_backward(X, W, mean, rstd)
         ctx.eps = eps
         ctx.bias_dtype = b.dtype if b is not None else None
-        return ops.layernorm(X, W, b, eps)
+        return y
 
     @staticmethod
     def backward(ctx, dY):
-        X, W = ctx.saved_tensors
+        X, W, mean, rstd = ctx.saved_tensors
         need_db = ctx.bias_dtype is not None and ctx.needs_input_grad[2]
         dx, dw, db = ops.layernorm_backward(dY, X, W, ctx.eps, need_dw=ctx.needs_input_grad[1],
-                                            need_db=need_db)
+                                            need_db=need_db, mean=mean, rstd=rstd)
         if db is not None and db.dtype != ctx.bias_dtype:
             db = db.to(ctx.bias_dtype)
         return dx, dw, db, None
@@ -98,15 +100,16 @@ class _ResidualRMSNormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, X, Residual, W, eps):
-        ctx.save_for_backward(X, Residual, W)
+        y, rstd = ops.residual_rmsnorm(X, Residual, W, eps, return_rstd=True)
+        ctx.save_for_backward(X, Residual, W, rstd)
         ctx.eps = eps
-        return ops.residual_rmsnorm(X, Residual, W, eps)
+        return y
 
     @staticmethod
     def backward(ctx, dY):
-        X, Residual, W = ctx.saved_tensors
+        X, Residual, W, rstd = ctx.saved_tensors
         dx, dw = ops.rmsnorm_backward(dY, X, W, ctx.eps, need_dw=ctx.needs_input_grad[2],
-                                      residual=Residual)
+                                      residual=Residual, rstd=rstd)
         return dx, dx, dw, None
 
 
@@ -116,17 +119,19 @@ class _ResidualLayerNormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, X, Residual, W, b, eps):
-        ctx.save_for_backward(X, Residual, W)
+        y, mean, rstd = ops.residual_layernorm(X, Residual, W, b, eps, return_stats=True)
+        ctx.save_for_backward(X, Residual, W, mean, rstd)
         ctx.eps = eps
         ctx.bias_dtype = b.dtype if b is not None else None
-        return ops.residual_layernorm(X, Residual, W, b, eps)
+        return y
 
     @staticmethod
     def backward(ctx, dY):
-        X, Residual, W = ctx.saved_tensors
+        X, Residual, W, mean, rstd = ctx.saved_tensors
         need_db = ctx.bias_dtype is not None and ctx.needs_input_grad[3]
         dx, dw, db = ops.layernorm_backward(dY, X, W, ctx.eps, need_dw=ctx.needs_input_grad[2],
-                                            need_db=need_db, residual=Residual)
+                                            need_db=need_db, residual=Residual, mean=mean,
+                                            rstd=rstd)
         if db is not None and db.dtype != ctx.bias_dtype:
             db = db.to(ctx.bias_dtype)
         return dx, dx, dw, db, None

@@ -93,9 +93,16 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
     return (y, rstd) if return_rstd else y
 
 
+def _row_stats(rows: int, dev: torch.device, mean: bool) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
+    """fp32 outputs for the row statistics: (mean or None, rstd)."""
+    return (torch.empty(rows, dtype=torch.float32, device=dev) if mean else None,
+            torch.empty(rows, dtype=torch.float32, device=dev))
+
+
 def layernorm(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[torch.Tensor],
-              eps: float = 1e-5) -> torch.Tensor:
-    """LayerNorm over the last dim; weight/bias may be None."""
+              eps: float = 1e-5, return_stats: bool = False):
+    """LayerNorm over the last dim; weight/bias may be None. With return_stats, (y, mean, rstd)
+    with the fp32 row statistics that layernorm_backward takes."""
     dev = _need_cuda(x, weight, bias)
     x2 = _rows(x)
     wb_dtype = weight.dtype if weight is not None else (bias.dtype if bias is not None else x.dtype)
@@ -105,14 +112,16 @@ def layernorm(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[to
         if t is not None and t.numel() != x.shape[-1]:
             raise ValueError("weight/bias size does not match the normalised dim")
     y = torch.empty((x2.shape[0], x2.shape[1]), dtype=x.dtype, device=dev)
+    mean, rstd = _row_stats(x2.shape[0], dev, True) if return_stats else (None, None)
     with torch.cuda.device(dev):
-        rc = _lib.load().trx_layernorm_fwd(_ptr(x2), _ptr(w), _ptr(b), _ptr(y), None, None,
+        rc = _lib.load().trx_layernorm_fwd(_ptr(x2), _ptr(w), _ptr(b), _ptr(y), _ptr(mean), _ptr(rstd),
                                            x2.shape[0], x2.shape[1], _row_stride(x2), x2.shape[1],
                                            float(eps), _code(x2), _DTYPE_CODE[wb_dtype],
                                            _stream(dev))
     _lib.check("trx_layernorm_fwd", rc)
     _count()
-    return y.view(x.shape)
+    y = y.view(x.shape)
+    return (y, mean, rstd) if return_stats else y
 
 
 # ----------------------------------------------------------------------------- int8
@@ -201,9 +210,9 @@ def rmsnorm_activation(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
 
 
 def residual_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor,
-                     eps: float = 1e-6, return_sum: bool = False):
+                     eps: float = 1e-6, return_sum: bool = False, return_rstd: bool = False):
     """RMSNorm(x + residual) with the sum kept in fp32 on chip; optionally also returns the
-    summed residual stream rounded to x's dtype."""
+    summed residual stream rounded to x's dtype, and the fp32 rstd that rmsnorm_backward takes."""
     dev = _need_cuda(x, residual, weight)
     if residual.shape != x.shape or residual.dtype != x.dtype:
         raise ValueError("residual must have the shape and dtype of x")
@@ -213,23 +222,27 @@ def residual_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tens
     w = weight.detach().contiguous()
     y = torch.empty((x2.shape[0], x2.shape[1]), dtype=x.dtype, device=dev)
     s = torch.empty_like(y) if return_sum else None
+    rstd = _row_stats(x2.shape[0], dev, False)[1] if return_rstd else None
     with torch.cuda.device(dev):
         rc = _lib.load().trx_residual_rmsnorm_fwd(
-            _ptr(x2), _ptr(r2), _ptr(w), _ptr(y), _ptr(s), None, x2.shape[0], x2.shape[1],
+            _ptr(x2), _ptr(r2), _ptr(w), _ptr(y), _ptr(s), _ptr(rstd), x2.shape[0], x2.shape[1],
             _row_stride(x2), _row_stride(r2), x2.shape[1], x2.shape[1], float(eps), _code(x2),
             _code(w), _stream(dev))
     _lib.check("trx_residual_rmsnorm_fwd", rc)
     _count()
-    y = y.view(x.shape)
-    return (y, s.view(x.shape)) if return_sum else y
+    out = (y.view(x.shape),)
+    out += (s.view(x.shape),) if return_sum else ()
+    out += (rstd,) if return_rstd else ()
+    return out if len(out) > 1 else out[0]
 
 
 def residual_layernorm(x: torch.Tensor, residual: torch.Tensor, weight: Optional[torch.Tensor],
                        bias: Optional[torch.Tensor], eps: float = 1e-5,
-                       return_sum: bool = False):
+                       return_sum: bool = False, return_stats: bool = False):
     """LayerNorm(x + residual) with the sum kept in fp32 on chip; the normalised value is rounded
     to x's dtype before the affine part, as the reference's fused module does. Optionally also
-    returns the summed residual stream rounded to x's dtype."""
+    returns the summed residual stream rounded to x's dtype, and the fp32 mean and rstd that
+    layernorm_backward takes."""
     dev = _need_cuda(x, residual, weight, bias)
     if residual.shape != x.shape or residual.dtype != x.dtype:
         raise ValueError("residual must have the shape and dtype of x")
@@ -242,15 +255,18 @@ def residual_layernorm(x: torch.Tensor, residual: torch.Tensor, weight: Optional
     x2, r2 = _rows(x), _rows(residual)
     y = torch.empty((x2.shape[0], x2.shape[1]), dtype=x.dtype, device=dev)
     s = torch.empty_like(y) if return_sum else None
+    mean, rstd = _row_stats(x2.shape[0], dev, True) if return_stats else (None, None)
     with torch.cuda.device(dev):
         rc = _lib.load().trx_residual_layernorm_fwd(
-            _ptr(x2), _ptr(r2), _ptr(w), _ptr(b), _ptr(y), _ptr(s), None, None, x2.shape[0],
+            _ptr(x2), _ptr(r2), _ptr(w), _ptr(b), _ptr(y), _ptr(s), _ptr(mean), _ptr(rstd), x2.shape[0],
             x2.shape[1], _row_stride(x2), _row_stride(r2), x2.shape[1], x2.shape[1], float(eps),
             _code(x2), _DTYPE_CODE[wb_dtype], _stream(dev))
     _lib.check("trx_residual_layernorm_fwd", rc)
     _count()
-    y = y.view(x.shape)
-    return (y, s.view(x.shape)) if return_sum else y
+    out = (y.view(x.shape),)
+    out += (s.view(x.shape),) if return_sum else ()
+    out += (mean, rstd) if return_stats else ()
+    return out if len(out) > 1 else out[0]
 
 
 def residual_rmsnorm_quantize(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor,
@@ -392,6 +408,12 @@ def glu_backward(dy: torch.Tensor, x: torch.Tensor, act: str) -> torch.Tensor:
     return dx.view(x.shape)
 
 
+def _stat(t: torch.Tensor, rows: int) -> torch.Tensor:
+    if t.dtype != torch.float32 or t.numel() != rows:
+        raise ValueError("row statistics must be float32, one per row")
+    return t.contiguous()
+
+
 def _norm_bwd_workspace(rows: int, cols: int, dev: torch.device) -> torch.Tensor:
     n = int(_lib.load().trx_norm_bwd_workspace_bytes(rows, cols))
     return torch.empty(n, dtype=torch.uint8, device=dev)
@@ -399,9 +421,10 @@ def _norm_bwd_workspace(rows: int, cols: int, dev: torch.device) -> torch.Tensor
 
 def rmsnorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
                      need_dw: bool = True, residual: Optional[torch.Tensor] = None,
-                     activation: Optional[str] = None):
+                     activation: Optional[str] = None, rstd: Optional[torch.Tensor] = None):
     """(dx, dw) of rmsnorm(x, weight, eps) given dy; dw is None when need_dw is False. The row
-    statistics are recomputed from x; dw is summed in fp32 in a fixed order. With `residual`, the
+    statistics are recomputed from x unless the forward's `rstd` is given (not with an
+    activation); dw is summed in fp32 in a fixed order. With `residual`, the
     gradient of residual_rmsnorm(x, residual, ...): dx is then also the residual's gradient. With
     `activation`, the gradient of rmsnorm_activation(x, weight, eps, activation)."""
     if activation is not None and activation not in ROW_ACTIVATIONS:
@@ -409,7 +432,9 @@ def rmsnorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, ep
                          f"Supported: {sorted(ROW_ACTIVATIONS)}")
     if activation is not None and residual is not None:
         raise ValueError("residual and activation cannot be combined")
-    dev = _need_cuda(dy, x, weight, residual)
+    if activation is not None and rstd is not None:
+        raise ValueError("rstd and activation cannot be combined")
+    dev = _need_cuda(dy, x, weight, residual, rstd)
     if dy.shape != x.shape or dy.dtype != x.dtype:
         raise ValueError("dy must have the shape and dtype of x")
     if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype):
@@ -430,6 +455,15 @@ def rmsnorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, ep
                 _row_stride(dy2), _row_stride(x2), x2.shape[1], float(eps),
                 ROW_ACTIVATIONS[activation], _code(x2), _code(w), _ptr(ws), ws.numel(),
                 _stream(dev))
+        elif rstd is not None:
+            name = "trx_rmsnorm_bwd_saved"
+            r2 = _rows(residual) if residual is not None else None
+            rstd = _stat(rstd, x2.shape[0])
+            rc = lib.trx_rmsnorm_bwd_saved(
+                _ptr(dy2), _ptr(x2), _ptr(r2), _ptr(w), _ptr(rstd), _ptr(dx), _ptr(dw), x2.shape[0],
+                x2.shape[1], _row_stride(dy2), _row_stride(x2),
+                _row_stride(r2) if r2 is not None else x2.shape[1], x2.shape[1], _code(x2), _code(w),
+                _ptr(ws), ws.numel(), _stream(dev))
         elif residual is None:
             name = "trx_rmsnorm_bwd"
             rc = lib.trx_rmsnorm_bwd(
@@ -450,11 +484,15 @@ def rmsnorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, ep
 
 def layernorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: Optional[torch.Tensor],
                        eps: float = 1e-5, need_dw: bool = True, need_db: bool = True,
-                       residual: Optional[torch.Tensor] = None):
+                       residual: Optional[torch.Tensor] = None,
+                       mean: Optional[torch.Tensor] = None, rstd: Optional[torch.Tensor] = None):
     """(dx, dw, db) of layernorm(x, weight, bias, eps) given dy; weight may be None (then dw is
-    None); db is returned in the weight's dtype (x's dtype without a weight). With `residual`,
+    None); db is returned in the weight's dtype (x's dtype without a weight). The row statistics
+    are recomputed from x unless the forward's `mean` and `rstd` are given. With `residual`,
     the gradient of residual_layernorm(x, residual, ...): dx is then also the residual's."""
-    dev = _need_cuda(dy, x, weight, residual)
+    dev = _need_cuda(dy, x, weight, residual, mean, rstd)
+    if (mean is None) != (rstd is None):
+        raise ValueError("mean and rstd come together")
     if dy.shape != x.shape or dy.dtype != x.dtype:
         raise ValueError("dy must have the shape and dtype of x")
     if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype):
@@ -471,7 +509,16 @@ def layernorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: Optional[torch
     ws = _norm_bwd_workspace(x2.shape[0], x2.shape[1], dev)
     lib = _lib.load()
     with torch.cuda.device(dev):
-        if residual is None:
+        if rstd is not None:
+            name = "trx_layernorm_bwd_saved"
+            r2 = _rows(residual) if residual is not None else None
+            mean, rstd = _stat(mean, x2.shape[0]), _stat(rstd, x2.shape[0])
+            rc = lib.trx_layernorm_bwd_saved(
+                _ptr(dy2), _ptr(x2), _ptr(r2), _ptr(w), _ptr(mean), _ptr(rstd), _ptr(dx), _ptr(dw),
+                _ptr(db), x2.shape[0], x2.shape[1], _row_stride(dy2), _row_stride(x2),
+                _row_stride(r2) if r2 is not None else x2.shape[1], x2.shape[1], _code(x2),
+                _DTYPE_CODE[p_dtype], _ptr(ws), ws.numel(), _stream(dev))
+        elif residual is None:
             name = "trx_layernorm_bwd"
             rc = lib.trx_layernorm_bwd(
                 _ptr(dy2), _ptr(x2), _ptr(w), _ptr(dx), _ptr(dw), _ptr(db), x2.shape[0],
