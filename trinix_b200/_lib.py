@@ -112,6 +112,10 @@ def lib_exists() -> bool:
     return os.path.exists(LIB_PATH)
 
 
+def loaded() -> bool:
+    return _lib is not None
+
+
 def load() -> ctypes.CDLL:
     """Load the shared library once; raise if it has not been built."""
     global _lib

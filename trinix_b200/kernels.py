@@ -23,7 +23,8 @@ from . import _lib, ops
 
 
 def _available() -> bool:
-    return torch.cuda.is_available() and _lib.lib_exists()
+    # a loaded library needs no look at the disk on every call
+    return torch.cuda.is_available() and (_lib.loaded() or _lib.lib_exists())
 
 
 class _ForwardOnly(torch.autograd.Function):
@@ -42,9 +43,11 @@ class _ForwardOnly(torch.autograd.Function):
 
 
 def _needs_graph(*args) -> bool:
-    return torch.is_grad_enabled() and any(
-        isinstance(a, torch.Tensor) and a.requires_grad for a in args
-    )
+    if torch.is_grad_enabled():
+        for a in args:
+            if isinstance(a, torch.Tensor) and a.requires_grad:
+                return True
+    return False
 
 
 def _run(fn, *args):
