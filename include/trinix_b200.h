@@ -395,6 +395,17 @@ int trx_attn_fwd_dropout(const void* q, const void* k, const void* v, void* out,
 int trx_attn_status(const void* workspace, unsigned int* host_word, void* stream);
 
 /*
+ * Attach a word of pinned host memory to an attention workspace (NULL detaches it; the workspace
+ * must have been zeroed before). From then on every launch on that workspace that gives up on a
+ * bounded wait, or that finds such a failure recorded and skips its work, also writes the status
+ * word there; a launch that works touches nothing. A host that reads the word before each call
+ * needs no trx_attn_status copies. The caller keeps the word alive as long as it is attached, and
+ * zeroes it together with the device word. One small launch on `stream`. Replaces nothing in the
+ * reference.
+ */
+int trx_attn_mirror(void* workspace, unsigned int* host_word_or_null, void* stream);
+
+/*
  * trx_attn_fwd for callers that cannot provide a workspace. No counterpart in the reference.
  *
  * Who needs it: hosts that pass pointers in but cannot create device memory when the call is

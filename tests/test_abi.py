@@ -89,6 +89,8 @@ def test_status_entry_point_validates_without_a_device(lib):
     word = ctypes.c_uint(0)
     assert lib.trx_attn_status(None, ctypes.byref(word), None) == -1
     assert lib.trx_attn_status(P(4096), None, None) == -1
+    assert lib.trx_attn_mirror(None, ctypes.byref(word), None) == -1
+    assert lib.trx_attn_mirror(P(4100), None, None) == -9
     word.value = 4  # a failure seen by an earlier copy: reported, nothing enqueued
     assert lib.trx_attn_status(P(4096), ctypes.byref(word), None) == -8
     assert word.value == 4

@@ -537,3 +537,21 @@ def test_dense_mask_at_every_alignment(cuda, Sk, D, dtype, wide):
         assert T.attention_status(cuda) == 0
         _, ref32 = _mask_ref(q, k, v, mask.float(), False)
         assert float((out.float().cpu() - ref32).abs().max()) <= TOL
+
+
+def test_recorded_failure_with_few_query_rows(cuda):
+    """The decode kernel too skips its work on a recorded failure and writes the host mirror; with
+    no failure the mirror stays untouched. The word is set from the host."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(1, 2, 700, 8, 2, 128, seed=3))
+    good = T.attention(q, k, v)
+    torch.cuda.synchronize(cuda)
+    assert int(ops._status_host[cuda.index or 0][0]) == 0
+    ops._workspace(cuda)[:4].view(torch.int32).fill_(4)
+    T.attention(q, k, v)
+    torch.cuda.synchronize(cuda)
+    assert int(ops._status_host[cuda.index or 0][0]) == 4
+    with pytest.raises(T._lib.TrinixB200Error):
+        T.attention(q, k, v)
+    assert torch.equal(T.attention(q, k, v), good)
+    assert T.attention_status(cuda) == 0

@@ -159,6 +159,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   atomicOr(status, code);
   return false;
 }
+// The status word's copy in host memory, if trx_attn_mirror attached one (workspace words 1 to 3:
+// a tag and the address). Written only by a launch that gave up or found a recorded failure, so a
+// launch that works pays nothing for it; a copy behind every launch, 4 bytes or not, holds the
+// stream for two hand-overs between the compute and the copy engine.
+constexpr unsigned ATT_MIRROR_TAG = 0x5452584du;
+__device__ __forceinline__ void report_status(unsigned int* status) {
+  if (status[1] != ATT_MIRROR_TAG) return;
+  volatile unsigned int* host = *reinterpret_cast<unsigned int* const*>(status + 2);
+  *host = *reinterpret_cast<volatile unsigned int*>(status);
+  __threadfence_system();
+}
+__global__ void attach_mirror_kernel(unsigned int* status, unsigned int* host) {
+  *reinterpret_cast<unsigned int**>(status + 2) = host;
+  status[1] = host ? ATT_MIRROR_TAG : 0u;
+}
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
                                             int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -500,6 +515,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   if (skip_launch) {  // nothing was started: give the TMEM columns back and leave
+    if (threadIdx.x == 0) report_status(p.status);
     if (warp == 0)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                    "r"(512u)
@@ -1140,6 +1156,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         }
         if (!done) atomicOr(p.status, ATT_ST_DRAIN);
       }
+    report_status(p.status);
   }
   __syncthreads();
   if (warp == 0) {
@@ -1408,6 +1425,19 @@ extern "C" int trx_attn_status(const void* workspace, unsigned int* host_word, v
                       static_cast<cudaStream_t>(stream)) != cudaSuccess)
     return TRX_ERR_CUDA;
   return TRX_OK;
+}
+
+extern "C" int trx_attn_mirror(void* workspace, unsigned int* host_word_or_null, void* stream) {
+  if (!workspace) return TRX_ERR_NULL_POINTER;
+  if (!aligned_to(workspace, 16)) return TRX_ERR_WORKSPACE;
+  void* dev = nullptr;
+  if (host_word_or_null && cudaHostGetDevicePointer(&dev, host_word_or_null, 0) != cudaSuccess) {
+    cudaGetLastError();  // not pinned memory: an error of this call, not of the next launch
+    return TRX_ERR_CUDA;
+  }
+  attach_mirror_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<unsigned int*>(workspace), static_cast<unsigned int*>(dev));
+  return cudaGetLastError() == cudaSuccess ? TRX_OK : TRX_ERR_CUDA;
 }
 
 extern "C" int trx_attn_fwd(const void* q, const void* k, const void* v, void* out,

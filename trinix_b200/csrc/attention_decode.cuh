@@ -282,6 +282,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
     }
   }
 
+  if ((!ok || skip) && lane == 0) report_status(p.status);
+
   // ---- this warp's partial result: O into its own ring, row maxima and sums beside it ----------
   float* ml = reinterpret_cast<float*>(smem + L::ML_OFF);        // [2][DEC_WARPS][ROWS]
   float* cta_ml = reinterpret_cast<float*>(smem + L::CTA_ML_OFF);  // [2][ROWS]

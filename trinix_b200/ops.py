@@ -75,8 +75,7 @@ def _launch(name: str, dev: torch.device, *args) -> None:
             rc = fn(*args, _raw_stream(index))
     if rc:
         _lib.check(name, rc)
-    if name != "trx_attn_status":  # a copy, not a kernel
-        _count()
+    _count()
 
 
 def _ptr(t: Optional[torch.Tensor]) -> int:
@@ -489,6 +488,9 @@ def _workspace(dev: torch.device) -> torch.Tensor:
         n = int(_lib.load().trx_attn_workspace_bytes())
         ws = torch.zeros(n, dtype=torch.uint8, device=torch.device("cuda", idx))
         host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        with torch.cuda.device(idx):
+            _lib.check("trx_attn_mirror", _lib.load().trx_attn_mirror(
+                ws.data_ptr(), host.data_ptr(), _raw_stream(idx)))
         _status_host[idx] = host
         _status_word[idx] = ctypes.c_int32.from_address(host.data_ptr())
         _workspaces[idx] = ws
@@ -496,10 +498,9 @@ def _workspace(dev: torch.device) -> torch.Tensor:
 
 
 def _raise_if_failed(fn: str, dev: torch.device) -> None:
-    """Host-side check of the status word's pinned mirror; no synchronisation. The mirror holds
-    what the copy queued behind the most recent COMPLETED launch saw. Non-zero: a kernel gave up
-    on a bounded wait, and it and every launch after it skipped their work, leaving their outputs
-    unwritten. Both copies of the word are cleared (so that the next call runs again) and the
+    """Host-side check of the status word's pinned mirror; no synchronisation. A kernel that gave up
+    on a bounded wait has written it, and so has every launch after it: they skipped their work and
+    left their outputs unwritten. Both copies of the word are cleared (so that the next call runs again) and the
     failure is raised; outputs returned since the failing launch must be discarded."""
     word = _status_word[_dev_index(dev)].value
     if word:
@@ -509,15 +510,6 @@ def _raise_if_failed(fn: str, dev: torch.device) -> None:
             fn, _lib.TRX_ERR_DEVICE_STATUS,
             f"{_lib.load().trx_status_string(_lib.TRX_ERR_DEVICE_STATUS).decode()} "
             f"(status word {word:#x}); attention outputs produced since then are invalid")
-
-
-def _queue_status_copy(ws: torch.Tensor, dev: torch.device) -> None:
-    index = _dev_index(dev)
-    try:
-        _launch("trx_attn_status", dev, ws.data_ptr(), _status_host[index].data_ptr())
-    except _lib.TrinixB200Error:  # the mirror turned non-zero while this call ran
-        _raise_if_failed("trx_attn_status", dev)
-        raise
 
 
 def attention_status(device=None) -> int:
@@ -647,5 +639,4 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool
         _launch("trx_attn_fwd_mask", dev, *head, *mask, *problem, *work)
     else:
         _launch("trx_attn_fwd", dev, *head, *problem, *work)
-    _queue_status_copy(ws, dev)
     return (out, lse) if return_lse else out
