@@ -367,3 +367,29 @@ def test_norm_backward_with_the_forwards_statistics(cuda, rows, cols, dtype):
             assert close(saved, again)
     with pytest.raises(ValueError):
         T.ops.rmsnorm_backward(dy, x, w, 1e-6, rstd=torch.ones(rows + 1, device=cuda))
+
+
+@pytest.mark.parametrize("nvec", [64, 65, 128, 129, 256, 257, 512, 513, 768, 769, 1024, 1025, 2048, 2049])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_norm_backward_at_the_edges_of_the_width_classes(cuda, nvec, dtype):
+    """Rows of the widest and narrowest width of every launch configuration (and the first one on
+    the scalar path), more rows than one CTA walks in some, statistics recomputed and saved: against
+    the float64 oracle within the bounds of the shape test (dx: one output rounding; dW and db: an
+    fp32 sum over the rows, then one rounding)."""
+    cols = nvec * (4 if dtype == torch.float32 else 8)
+    rows = 40
+    g = torch.Generator().manual_seed(nvec)
+    x, dy = (torch.randn(rows, cols, generator=g).to(dtype) for _ in range(2))
+    w, b = (torch.randn(cols, generator=g).to(dtype) for _ in range(2))
+    xc, dyc, wc, bc = (t.to(cuda) for t in (x, dy, w, b))
+    rx, rw = R.autograd_ref(lambda a, ww: R.rmsnorm_ref(a, ww, 1e-6), _f(x, w), dy.double())
+    lx, lw, lb = R.autograd_ref(lambda a, ww, bb: R.layernorm_ref(a, ww, bb, 1e-5), _f(x, w, b), dy.double())
+    _, rstd = T.ops.rmsnorm(xc, wc, 1e-6, return_rstd=True)
+    _, mean, ln_rstd = T.ops.layernorm(xc, wc, bc, 1e-5, return_stats=True)
+    tol, tol_sum = TOL32[dtype], max(TOL32[dtype], 1e-4)
+    for kw_r, kw_l in (({}, {}), ({"rstd": rstd}, {"mean": mean, "rstd": ln_rstd})):
+        dx, dw = T.ops.rmsnorm_backward(dyc, xc, wc, 1e-6, **kw_r)
+        assert rel_err(dx.cpu().double(), rx) <= tol and rel_err(dw.cpu().double(), rw) <= tol_sum
+        dx, dw, db = T.ops.layernorm_backward(dyc, xc, wc, 1e-5, **kw_l)
+        assert rel_err(dx.cpu().double(), lx) <= tol and rel_err(dw.cpu().double(), lw) <= tol_sum
+        assert rel_err(db.cpu().double(), lb) <= tol_sum

@@ -1,6 +1,6 @@
 // Backward of the row and gate ops: RMSNorm, LayerNorm (dx, dW, db) and the three GLUs.
 //
-// Norms. A CTA of 128 to 512 threads walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; a row of x and
+// Norms. A CTA of 64 to 512 threads walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; a row of x and
 // of dy is read from HBM once with 128-bit streaming loads and stays in registers. The row's
 // statistics are the forward's (SAVED) or recomputed from x; what bounds the kernel is the latency
 // of the CTA-wide reductions of a row at 12 to 24 warps per SM, and the saved statistics leave one
@@ -10,7 +10,7 @@
 // second kernel adds the P rows in a fixed order: dW and db are deterministic for a given shape
 // and device. (The reference accumulates dW across programs under spin locks,
 // kernels/rmsnorm_kernel.py:65-150, so its summation order changes from run to run.)
-// Rows that do not fit the vector path (odd widths, unaligned pointers, more than 1024 vectors)
+// Rows that do not fit the vector path (odd widths, unaligned pointers, more than 2048 vectors)
 // take scalar multi-pass kernels: dx plus per-row (mean, rstd) into the workspace, then column
 // sums over row slices into the same (P, C) block.
 //
@@ -19,22 +19,9 @@
 // written straight into the halves of a concatenated (R, 2H) gradient.
 #include "common.cuh"
 
-// RMSNorm: vectors per thread for rows of 257..512 vectors (512 / this many threads per row)
-#ifndef TRX_BWD512_VPT
-#define TRX_BWD512_VPT 2
-#endif
 // rows ahead of the current one that a CTA asks the copy engine to pull into L2 (0 = off)
 #ifndef TRX_BWD_L2_PREFETCH
 #define TRX_BWD_L2_PREFETCH 1
-#endif
-// minimum resident CTAs (of up to 256 threads) per SM asked of the compiler (caps registers per thread);
-// without it the compiler spends registers freely and the occupancy drops (measured: LayerNorm
-// 336 us at 121 registers, 208 us at 80)
-#ifndef TRX_BWD_MINB_LN
-#define TRX_BWD_MINB_LN 3
-#endif
-#ifndef TRX_BWD_MINB_RMS
-#define TRX_BWD_MINB_RMS 3
 #endif
 // grid of the norm backward kernel in resident waves
 #ifndef TRX_BWD_WAVES
@@ -122,9 +109,10 @@ __device__ __forceinline__ float act_grad(int act, float z) {
   return 2.0f * fmaxf(z, 0.0f);
 }
 
-template <bool LN, bool SAVED, typename T, int VPT, int NT>
-__global__ void __launch_bounds__(NT, NT <= 256 ? (LN ? TRX_BWD_MINB_LN : TRX_BWD_MINB_RMS) : 1)
-    norm_bwd_kernel(const NormBwdParams p) {
+// MIN_CTAS: resident CTAs per SM asked of the compiler (caps the registers per thread; without it
+// the compiler spends them freely and the occupancy drops).
+template <bool LN, bool SAVED, typename T, int VPT, int NT, int MIN_CTAS>
+__global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdParams p) {
   using P = Pack<T>;
   constexpr int VEC = P::VEC;
   __shared__ float2 red[2][NT / 32];
@@ -435,7 +423,7 @@ static int64_t norm_bwd_partial_rows(int64_t R, int64_t C) {
 
 // TRX_BWD_WAVES resident waves of CTAs (each walks R / grid rows); P_rows comes back as the grid size, i.e.
 // the number of rows of partial sums that were written.
-template <bool LN, bool SAVED, typename T, int VPT, int NT>
+template <bool LN, bool SAVED, typename T, int VPT, int NT, int MIN_CTAS>
 static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStream_t stream) {
   static std::atomic<int> blocks_per_sm_of[64];  // racing first calls store the same value
   int dev = 0;
@@ -444,7 +432,7 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   int blocks_per_sm = cacheable ? blocks_per_sm_of[dev].load(std::memory_order_acquire) : 0;
   if (blocks_per_sm == 0) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, SAVED, T, VPT, NT>, NT, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, SAVED, T, VPT, NT, MIN_CTAS>, NT, 0) !=
             cudaSuccess || n <= 0)
       n = 1;
     blocks_per_sm = n;
@@ -452,26 +440,38 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   }
   const int64_t resident = static_cast<int64_t>(sm_count_of_current_device()) * blocks_per_sm * TRX_BWD_WAVES;
   if (P_rows > resident) P_rows = resident;
-  norm_bwd_kernel<LN, SAVED, T, VPT, NT><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
+  norm_bwd_kernel<LN, SAVED, T, VPT, NT, MIN_CTAS><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
 }
 
 template <bool LN, bool SAVED, typename T>
 static void launch_norm_bwd_width(const NormBwdParams& p, int64_t nvec, int64_t& P_rows,
                                   cudaStream_t stream) {
-  // few vectors per thread: the running column sums cost 8 (16 for LayerNorm) registers each
-  if (nvec <= 256) {
-    launch_norm_bwd_vec<LN, SAVED, T, 1, 256>(p, P_rows, stream);
-  } else if (nvec <= 512) {
-    // measured on 32768 x 4096 bf16, statistics recomputed: RMSNorm 256 threads x 2 vectors (146
-    // us; 159 us at 128 x 4), LayerNorm 128 x 4 (170 us; 188 us at 256 x 2): LayerNorm then has
-    // three CTA-wide reductions per row, which four warps finish sooner than eight; 512 threads x
-    // 1 vector is slower for both (213 / 278 us). With the forward's statistics, one reduction:
-    // RMSNorm 136.4 us (156 / 234 us at 2 / 4 CTAs per SM), LayerNorm 151.5 us at 128 x 4 (163.5 us
-    // at 256 x 2; 175.6 / 218.8 us at 2 / 4 CTAs per SM)
-    constexpr int V = LN ? 4 : TRX_BWD512_VPT;
-    launch_norm_bwd_vec<LN, SAVED, T, V, 512 / V>(p, P_rows, stream);
+  // A row's threads meet in CTA-wide reductions, so few warps per row and many CTAs per SM are what
+  // hides them, until the running column sums (8 registers per vector and thread, 16 for LayerNorm)
+  // fill the register file. (vectors per thread, threads, CTAs per SM), measured in us with the
+  // forward's statistics, LayerNorm / RMSNorm, bf16 unless noted:
+  //   32768 x 512   (1, 64, 12) 39.2 / 37.0    (1, 256, 3) 70.1 / 55.4
+  //   32768 x 768   (1, 128, 6) 49.1 / 41.4    (1, 256, 3) 73.9 / 58.8
+  //   32768 x 2048  (2, 128, 5) 82.7 / 73.5    (1, 256, 3) 96.5 / 79.3    (4, 64, 6) 82.8 / 80.6
+  //   32768 x 1024 fp32         75.0 / 72.5                76.4 / 70.3
+  //   32768 x 4096  (4, 128, 3) 151.5 / 135.6  (2, 256, 3) 163.5 / 136.4  (4, 128, 4) 218.8 / -
+  //   8192 x 5120   (3, 256, 2) 62.4 / 59.2    (2, 512, 1) 86.8 / 82.1    (2, 384, 1) 80.1 / 76.8
+  //   8192 x 8192   (2, 512, 1) 102.6 / 94.9   (4, 256, 2) 119.2 / 79.2
+  //   8192 x 4096 fp32          88.1 / 85.7                73.1 / 73.6
+  //   8192 x 12288  (4, 512, 1) 213.7 / 129.8  (2, 1024, 1) 262.2 / 198.6  scalar path 875 / 831
+  //   8192 x 5120 fp32          107.2 / 104.4               125.0 / 117.5              387 / 356
+  constexpr bool F32 = Pack<T>::VEC == 4;
+  constexpr int V256 = LN || !F32 ? 2 : 1;
+  if (nvec <= 64) launch_norm_bwd_vec<LN, SAVED, T, 1, 64, 12>(p, P_rows, stream);
+  else if (nvec <= 128) launch_norm_bwd_vec<LN, SAVED, T, 1, 128, 6>(p, P_rows, stream);
+  else if (nvec <= 256) launch_norm_bwd_vec<LN, SAVED, T, V256, 256 / V256, V256 == 2 ? 5 : 3>(p, P_rows, stream);
+  else if (nvec <= 512) launch_norm_bwd_vec<LN, SAVED, T, LN ? 4 : 2, LN ? 128 : 256, 3>(p, P_rows, stream);
+  else if (nvec <= 768) launch_norm_bwd_vec<LN, SAVED, T, 3, 256, 2>(p, P_rows, stream);
+  else if (nvec <= 1024) {
+    if constexpr (LN && !F32) launch_norm_bwd_vec<LN, SAVED, T, 2, 512, 1>(p, P_rows, stream);
+    else launch_norm_bwd_vec<LN, SAVED, T, 4, 256, 2>(p, P_rows, stream);
   } else {
-    launch_norm_bwd_vec<LN, SAVED, T, 2, 512>(p, P_rows, stream);
+    launch_norm_bwd_vec<LN, SAVED, T, 4, 512, 1>(p, P_rows, stream);
   }
 }
 
@@ -491,7 +491,7 @@ static int launch_norm_bwd(NormBwdParams p, void* dw, void* db, float* ws, cudaS
     if (p.w) vec_ok = vec_ok && aligned_to(p.w, 16);
     if (p.res) vec_ok = vec_ok && aligned_to(p.res, 16) && (p.res_stride % VEC == 0);
     const int64_t nvec = p.C / VEC;
-    if (vec_ok && nvec <= 1024) {
+    if (vec_ok && nvec <= 2048) {
       if (p.rstd) launch_norm_bwd_width<LN, true, T>(p, nvec, P_rows, stream);
       else launch_norm_bwd_width<LN, false, T>(p, nvec, P_rows, stream);
     } else {
