@@ -405,6 +405,24 @@ def test_views_the_tensor_maps_cannot_take_are_materialised(cuda):
     assert torch.equal(out, T.triton_attn_func(*(odd.contiguous(),) * 3))
 
 
+@pytest.mark.parametrize("shape,strides", [
+    ((2, 5, 1, 64), (320, 64, 1, 1)),            # one head, few rows
+    ((2, 300, 1, 64), (19200, 64, 1, 1)),        # one head, many rows
+    ((1, 1, 8, 128), (3077, 3077, 128, 1)),      # one row of one sequence
+    ((1, 200, 8, 128), (204803, 1024, 128, 1)),  # one sequence
+    ((3, 1, 8, 128), (1024, 7, 128, 1)),         # one row each
+])
+def test_size_one_dims_of_any_stride(cuda, shape, strides):
+    """The stride of a size-1 dim addresses nothing, whatever its value."""
+    g = torch.Generator().manual_seed(shape[1])
+    q = torch.randn(204803, generator=g).bfloat16().to(cuda).as_strided(shape, strides)
+    out = T.triton_attn_func(q, q, q, causal=True)
+    assert out.stride() == torch.empty(shape).stride()
+    assert torch.equal(out, T.triton_attn_func(*(q.clone(memory_format=torch.contiguous_format),) * 3,
+                                               causal=True))
+    assert T.attention_status(cuda) == 0
+
+
 def test_flash_stand_in_keeps_the_conventions_of_the_symbol_it_replaces(cuda):
     """flash_attn_func (the symbol bound at trinix/layers/attention/base.py:10-16): causal with
     Sq < Sk is aligned bottom-right (decode against a KV cache sees every cached key), unknown

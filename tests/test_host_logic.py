@@ -195,3 +195,17 @@ def test_fuse_registry_mirrors_the_reference_contract():
         fused(torch.zeros(2, 8))
     with pytest.raises(ValueError, match="CUDA"):   # no CPU path behind the fused module
         fused(torch.zeros(2, 4096))
+
+
+@pytest.mark.parametrize("shape,strides", [
+    ((2, 5, 1, 64), (320, 64, 1, 1)),     # one head: unsqueeze(-1).transpose(2, 3)
+    ((1, 1, 8, 128), (3077, 3077, 128, 1)),
+    ((3, 1, 8, 128), (1024, 7, 128, 1)),
+    ((2, 4, 6), (48, 12, 2)),             # not contiguous at all
+])
+def test_outputs_have_the_strides_of_a_contiguous_tensor(shape, strides):
+    """Whatever strides the input's size-1 dims carry: the entry points test their outputs'."""
+    from trinix_b200 import ops
+    x = torch.empty(4 * 3077).as_strided(shape, strides)
+    assert ops._new(x).stride() == torch.empty(shape).stride()
+    assert ops._new(x, torch.int8).dtype == torch.int8
