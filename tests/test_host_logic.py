@@ -209,3 +209,16 @@ def test_outputs_have_the_strides_of_a_contiguous_tensor(shape, strides):
     x = torch.empty(4 * 3077).as_strided(shape, strides)
     assert ops._new(x).stride() == torch.empty(shape).stride()
     assert ops._new(x, torch.int8).dtype == torch.int8
+
+
+def test_outputs_are_plain_tensors_for_any_tensor_type():
+    from trinix_b200 import ops
+
+    class Tagged(torch.Tensor):
+        pass
+
+    x = torch.ones(3, 8, dtype=torch.bfloat16)
+    for t in (x, torch.nn.Parameter(x), x.as_subclass(Tagged), x.as_subclass(Tagged).t()):
+        for out in (ops._new(t), ops._empty(t, t.shape)):
+            assert type(out) is torch.Tensor and not out.requires_grad
+            assert out.shape == t.shape and out.dtype == x.dtype and out.is_contiguous()

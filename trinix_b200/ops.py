@@ -100,12 +100,25 @@ def _rows(x: torch.Tensor) -> Tuple[torch.Tensor, int, int]:
     return x2, x2.shape[0], x2.stride(0) if x2.shape[0] > 1 else c
 
 
+# Types whose empty_like / new_empty are plain tensors; for any other subclass they are instances of it.
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _empty(x: torch.Tensor, shape, dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    """An uninitialised plain tensor on x's device, of x's dtype unless another one is given."""
+    if type(x) in _PLAIN:
+        return x.new_empty(shape, dtype=dtype)
+    return torch.empty(shape, dtype=dtype or x.dtype, device=x.device)
+
+
 def _new(x: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """An uninitialised tensor of x's shape with the strides of a contiguous one. Without the memory
+    """The same of x's shape, with the strides of a contiguous tensor. Without the memory
     format empty_like keeps x's strides, arbitrary ones of size-1 dims among them, which the C
     entries that check their output's strides refuse. (1.0 us of host time; torch.empty with a
     dtype and a device 3.6.)"""
-    return torch.empty_like(x, dtype=dtype, memory_format=torch.contiguous_format)
+    if type(x) in _PLAIN:
+        return torch.empty_like(x, dtype=dtype, memory_format=torch.contiguous_format)
+    return _empty(x, x.shape, dtype)
 
 
 def _check_weight(weight: torch.Tensor, x: torch.Tensor) -> None:
@@ -129,7 +142,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
 
 def _row_stat(x: torch.Tensor, rows: int) -> torch.Tensor:
     """fp32 output for one statistic per row of x."""
-    return x.new_empty(rows, dtype=torch.float32)
+    return _empty(x, rows, dtype=torch.float32)
 
 
 def _affine(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[torch.Tensor]):
@@ -163,7 +176,7 @@ def quantize_rowwise(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     dev = _need_cuda(x)
     x2, rows, stride = _rows(x)
     c, codes = x.shape[-1], _new(x, torch.int8)
-    scales = x.new_empty(x.shape[:-1], dtype=torch.float32)
+    scales = _empty(x, x.shape[:-1], dtype=torch.float32)
     _launch("trx_quant_rowwise_i8", dev, x2.data_ptr(), codes.data_ptr(), scales.data_ptr(), rows, c,
             stride, c, _code(x2))
     return codes, scales
@@ -199,7 +212,7 @@ def rmsnorm_quantize(x: torch.Tensor, weight: torch.Tensor,
     _check_weight(weight, x)
     x2, rows, stride = _rows(x)
     w, c, codes = _dense(weight), x.shape[-1], _new(x, torch.int8)
-    scales = x.new_empty(x.shape[:-1], dtype=torch.float32)
+    scales = _empty(x, x.shape[:-1], dtype=torch.float32)
     _launch("trx_rmsnorm_quant_i8", dev, x2.data_ptr(), w.data_ptr(), codes.data_ptr(),
             scales.data_ptr(), rows, c, stride, c, float(eps), _code(x2), _code(w))
     return codes, scales
@@ -275,7 +288,7 @@ def residual_rmsnorm_quantize(x: torch.Tensor, residual: torch.Tensor, weight: t
     _check_weight(weight, x)
     (x2, rows, stride), (r2, _, r_stride) = _rows(x), _rows(residual)
     w, c, codes = _dense(weight), x.shape[-1], _new(x, torch.int8)
-    scales = x.new_empty(x.shape[:-1], dtype=torch.float32)
+    scales = _empty(x, x.shape[:-1], dtype=torch.float32)
     s = _new(x) if return_sum else None
     _launch("trx_residual_rmsnorm_quant_i8", dev, x2.data_ptr(), r2.data_ptr(), w.data_ptr(),
             codes.data_ptr(), scales.data_ptr(), _ptr(s), rows, c, stride, r_stride, c, c, float(eps),
@@ -341,7 +354,7 @@ def glu(x: torch.Tensor, act: str) -> torch.Tensor:
         raise ValueError("last dimension must be even")
     h = two_h // 2
     x2, rows, stride = _rows(x)
-    y = x.new_empty((*x.shape[:-1], h))
+    y = _empty(x, (*x.shape[:-1], h))
     up = x2.data_ptr()
     _launch("trx_glu_fwd", dev, up, up + h * x2.element_size(), y.data_ptr(), rows, h, stride, stride, h,
             GLU_ACTS[act], _code(x2))
@@ -384,7 +397,7 @@ def _stat(t: torch.Tensor, rows: int) -> torch.Tensor:
 
 
 def _norm_bwd_workspace(x: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
-    return x.new_empty(_lib.load().trx_norm_bwd_workspace_bytes(rows, cols), dtype=torch.uint8)
+    return _empty(x, _lib.load().trx_norm_bwd_workspace_bytes(rows, cols), dtype=torch.uint8)
 
 
 def rmsnorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
@@ -452,8 +465,8 @@ def layernorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: Optional[torch
     r2, _, r_stride = _rows(residual) if residual is not None else (None, 0, x.shape[-1])
     w, c, dx = _dense(weight), x.shape[-1], _new(x)
     p_dtype = w.dtype if w is not None else x.dtype
-    dw = w.new_empty(c) if need_dw and w is not None else None
-    db = x.new_empty(c, dtype=p_dtype) if need_db else None
+    dw = _empty(w, c) if need_dw and w is not None else None
+    db = _empty(x, c, dtype=p_dtype) if need_db else None
     ws = _norm_bwd_workspace(x, rows, c)
     tail = (_code(x2), _DTYPE_CODE[p_dtype], ws.data_ptr(), ws.numel())
     if rstd is not None:
@@ -615,7 +628,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool
         if slopes.numel() != Hq:
             raise ValueError(f"alibi_slopes must have {Hq} entries")
     out = _new(q)
-    lse = q.new_empty((B, Hq, Sq), dtype=torch.float32) if return_lse else None
+    lse = _empty(q, (B, Hq, Sq), dtype=torch.float32) if return_lse else None
     ws = _workspace(dev)
     # a failure recorded by an earlier launch surfaces here, before more work is queued
     _raise_if_failed("trx_attn_fwd", dev)
