@@ -1,6 +1,8 @@
 """Parity of the tcgen05 attention kernel with the CPU oracle (the reference's PyTorch
 attention), through triton_attn_func / the C ABI. Tolerance from the project baseline:
 2e-2 max abs error in bf16."""
+import ctypes
+
 import pytest
 import torch
 
@@ -573,3 +575,41 @@ def test_recorded_failure_with_few_query_rows(cuda):
         T.attention(q, k, v)
     assert torch.equal(T.attention(q, k, v), good)
     assert T.attention_status(cuda) == 0
+
+
+@pytest.mark.parametrize("B,Sq,Sk", [(16, 1, 4093), (40, 2, 3000), (1, 4, 20000), (64, 1, 300)])
+def test_few_query_rows_while_a_failure_is_being_recorded(cuda, B, Sq, Sk):
+    """The status word may turn non-zero while a launch runs (a launch on another stream gives up).
+    Warps, CTAs and the CTAs of a cluster then read different values: every output row is either
+    the whole result or untouched, never a sum of some of the parts. The word is written by a copy
+    from the host beside the launch, at several distances; no wait is made to run out."""
+    q, k, v = (t.to(cuda) for t in _qkv(B, Sq, Sk, 32, 8, 128, seed=B))
+    good = T.attention(q, k, v)
+    lib = T._lib.load()
+    P, st3 = ctypes.c_void_p, T._lib.I64x3
+    ws = torch.zeros(256, dtype=torch.uint8, device=cuda)
+    word = torch.full((1,), 4, dtype=torch.int32).pin_memory()
+    side, main = torch.cuda.Stream(cuda), torch.cuda.current_stream(cuda)
+    mixed = 0
+    for trial in range(60):
+        ws.zero_()
+        out = torch.full_like(q, 7.0)
+        lse = torch.full((B, 32, Sq), 7.0, device=cuda)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1500 * trial)  # 0 to 50 us
+            ws[:4].view(torch.int32).copy_(word, non_blocking=True)
+        assert lib.trx_attn_fwd(
+            P(q.data_ptr()), P(k.data_ptr()), P(v.data_ptr()), P(out.data_ptr()), P(lse.data_ptr()),
+            None, B, Sq, Sk, 32, 8, 128, st3(*q.stride()[:3]), st3(*k.stride()[:3]),
+            st3(*v.stride()[:3]), st3(*out.stride()[:3]), 128 ** -0.5, 0, -1, -1, 2,
+            P(ws.data_ptr()), 256, P(main.cuda_stream)) == 0
+        torch.cuda.synchronize(cuda)
+        same = (out == good).all(-1)
+        untouched = (out == 7.0).all(-1)
+        assert bool((same | untouched).all())
+        assert torch.equal((lse == 7.0).transpose(1, 2), untouched)
+        mixed += bool(same.any()) and bool(untouched.any())
+    # nothing left over: the launch after it works
+    assert torch.equal(T.attention(q, k, v), good) and T.attention_status(cuda) == 0
+    print(f"{mixed} of 60 launches caught half way")

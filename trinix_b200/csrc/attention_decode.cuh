@@ -43,7 +43,7 @@ struct DecSmem {
   static constexpr int ML_OFF = BAR_OFF + DEC_WARPS * DEC_STAGES * 8;  // max, sum per warp and row
   static constexpr int CTA_ML_OFF = ML_OFF + 2 * DEC_WARPS * ROWS * 4;
   static constexpr int FLAG_OFF = CTA_ML_OFF + 2 * ROWS * 4;
-  static constexpr int TOTAL = FLAG_OFF + DEC_WARPS * 4;
+  static constexpr int TOTAL = FLAG_OFF + (DEC_WARPS + 1) * 4;  // a flag per warp, one of the CTA
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for 1024-byte alignment
 };
 
@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
 
   const uint32_t ring = sbase + warp * L::RING_BYTES;
   const uint32_t bars = sbase + L::BAR_OFF + warp * DEC_STAGES * 8;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::FLAG_OFF) + warp;
+  int* no_result = reinterpret_cast<int*>(smem + L::FLAG_OFF);  // [DEC_WARPS], then the CTA's
+  volatile int* abort_flag = no_result + warp;
   const int kh = h0 / p.k_hdiv, vh = h0 / p.v_hdiv, kb = b * p.k_bmul, vb = b * p.v_bmul;
   auto issue_fill = [&](int it) {  // one lane: K and V of the it-th tile of this warp
     const int s = it % DEC_STAGES, key0 = (first + it * DEC_WARPS) * DEC_KEYS;
@@ -139,8 +140,12 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
     for (int it = 0; it < min(n_it, DEC_STAGES); ++it) issue_fill(it);
   }
   __syncwarp();
-  // A launch that follows a recorded failure writes nothing; the copies above are waited for.
-  const bool skip = *reinterpret_cast<volatile unsigned int*>(p.status) != 0u;
+  // A launch that follows a recorded failure writes nothing; the copies above are waited for. The
+  // word may turn non-zero at any time (another CTA, another stream), so one lane reads it for its
+  // warp, whose trip count depends on it; what the other warps and CTAs read is settled at the end.
+  unsigned int seen = 0;
+  if (lane == 0) seen = *reinterpret_cast<volatile unsigned int*>(p.status);
+  const bool skip = __shfl_sync(0xffffffffu, seen, 0) != 0u;
   if (skip) n_it = min(n_it, DEC_STAGES);
 
   // Q as mma A fragments: rows rl and rl + 8 of each 16-row tile
@@ -276,15 +281,21 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
   if (!ok) {  // gave up on tile `it`: wait (bounded) for the copies still in flight
     for (int f = it; f < min(n_it, it + DEC_STAGES); ++f) {
       const uint64_t t0 = global_ns();
-      while (!mbar_try_wait(bars + 8 * (f % DEC_STAGES), (f / DEC_STAGES) & 1) &&
-             global_ns() - t0 < ATT_WAIT_NS) {
-      }
+      bool done = false;
+      while (!done && global_ns() - t0 < ATT_WAIT_NS)
+        done = mbar_try_wait(bars + 8 * (f % DEC_STAGES), (f / DEC_STAGES) & 1);
+      if (!done) atomicOr(p.status, ATT_ST_DRAIN);
     }
+    __syncwarp();  // lane 0 reports what every lane has recorded
+  }
+  const bool has_result = ok && !skip;
+  if (!has_result && lane == 0) {
+    *abort_flag = 1;
+    report_status(p.status);
   }
 
-  if ((!ok || skip) && lane == 0) report_status(p.status);
-
   // ---- this warp's partial result: O into its own ring, row maxima and sums beside it ----------
+  // (not from a warp without one: a copy that was given up may still be writing the ring)
   float* ml = reinterpret_cast<float*>(smem + L::ML_OFF);        // [2][DEC_WARPS][ROWS]
   float* cta_ml = reinterpret_cast<float*>(smem + L::CTA_ML_OFF);  // [2][ROWS]
   float* ow = reinterpret_cast<float*>(smem + warp * L::RING_BYTES);
@@ -301,19 +312,22 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
         ml[warp * L::ROWS + r] = m_run[m][e];
         ml[(DEC_WARPS + warp) * L::ROWS + r] = l;
       }
-      if (r0 + r < rows)
+      if (has_result && r0 + r < rows)
 #pragma unroll
         for (int n = 0; n < D / 8; ++n)
           *reinterpret_cast<float2*>(ow + r * D + 8 * n + 2 * q4) =
               make_float2(o[m][n][2 * e], o[m][n][2 * e + 1]);
     }
   __syncthreads();
+  bool whole = true;  // every warp (below: of the cluster) has a result; else nothing is written
+#pragma unroll
+  for (int w = 0; w < DEC_WARPS; ++w) whole = whole && no_result[w] == 0;
 
   // out[row, 4 c4 ..] = acc / l, and the row's LSE
   auto emit = [&](int r, int c4, float4 acc, float mx, float l) {
     const int s = (r0 + r) / group, h = h0 + (r0 + r) % group;
     const float inv = l > 0.0f ? __fdividef(1.0f, l) : 0.0f;
-    if (!skip) {
+    if (whole) {
       uint2 v;
       v.x = pack16<BF16>(acc.x * inv, acc.y * inv);
       v.y = pack16<BF16>(acc.z * inv, acc.w * inv);
@@ -356,8 +370,12 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
     }
   }
   if (nsplit == 1) return;
+  if (threadIdx.x == 0) no_result[DEC_WARPS] = whole ? 0 : 1;
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
+  static_assert(DEC_MAX_SPLIT <= 32, "one lane per CTA");
+  whole = __all_sync(0xffffffffu, lane >= nsplit ||
+                                      cluster.map_shared_rank(no_result, lane)[DEC_WARPS] == 0);
   for (int idx = split * DEC_THREADS + threadIdx.x; idx < live_rows * (D / 4);
        idx += nsplit * DEC_THREADS) {
     const int r = idx / (D / 4), c4 = idx % (D / 4);
