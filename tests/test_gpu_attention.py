@@ -613,3 +613,25 @@ def test_few_query_rows_while_a_failure_is_being_recorded(cuda, B, Sq, Sk):
     # nothing left over: the launch after it works
     assert torch.equal(T.attention(q, k, v), good) and T.attention_status(cuda) == 0
     print(f"{mixed} of 60 launches caught half way")
+
+
+def test_recorded_failure_is_raised_once_with_calls_in_flight(cuda):
+    """Launches that were queued before the host saw the failure skip their work and report it too,
+    possibly after it was raised: that report belongs to the same failure."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(1, 300, 300, 4, 2, 128, seed=13))
+    good = T.attention(q, k, v)
+    torch.cuda.synchronize(cuda)
+    ops._workspace(cuda)[:4].view(torch.int32).fill_(4)
+    T.attention(q, k, v)
+    seen = torch.cuda.Event()
+    seen.record()
+    torch.cuda._sleep(40_000_000)  # some 20 ms
+    T.attention(q, k, v)           # queued behind it: reports once more
+    seen.synchronize()
+    with pytest.raises(T._lib.TrinixB200Error):
+        T.attention(q, k, v)
+    for _ in range(3):
+        assert torch.equal(T.attention(q, k, v), good)
+        torch.cuda.synchronize(cuda)
+    assert T.attention_status(cuda) == 0

@@ -510,15 +510,25 @@ def _workspace(dev: torch.device) -> torch.Tensor:
     return ws
 
 
+def _clear_status(dev: torch.device) -> None:
+    """Zero both copies of the status word. Launches queued before the device's copy is cleared still
+    find the failure and write the host's copy, so that one is cleared when none of them is left."""
+    _workspace(dev)[:4].zero_()
+    torch.cuda.synchronize(dev)
+    _status_host[_dev_index(dev)].zero_()
+
+
 def _raise_if_failed(fn: str, dev: torch.device) -> None:
-    """Host-side check of the status word's pinned mirror; no synchronisation. A kernel that gave up
-    on a bounded wait has written it, and so has every launch after it: they skipped their work and
-    left their outputs unwritten. Both copies of the word are cleared (so that the next call runs again) and the
-    failure is raised; outputs returned since the failing launch must be discarded."""
+    """Host-side check of the status word's pinned mirror; no synchronisation while it is zero. A
+    kernel that gave up on a bounded wait has written it, and so has every launch after it: they
+    skipped their work and left their outputs unwritten. Both copies of the word are cleared, behind
+    whatever is in flight, and the failure is raised: once, and the next call runs again (under
+    stream capture, where nothing can be waited for, it is raised and stays). Outputs returned since
+    the failing launch must be discarded."""
     word = _status_word[_dev_index(dev)].value
     if word:
-        _workspace(dev)[:4].zero_()
-        _status_host[_dev_index(dev)].zero_()
+        if not torch.cuda.is_current_stream_capturing():
+            _clear_status(dev)
         raise _lib.TrinixB200Error(
             fn, _lib.TRX_ERR_DEVICE_STATUS,
             f"{_lib.load().trx_status_string(_lib.TRX_ERR_DEVICE_STATUS).decode()} "
@@ -532,9 +542,9 @@ def attention_status(device=None) -> int:
     ws = _workspace(dev)
     word = int(ws[:4].view(torch.int32).item())  # .item() waits for the stream
     if word:
-        ws[:4].zero_()
-    torch.cuda.current_stream(dev).synchronize()
-    _status_host[_dev_index(dev)].zero_()
+        _clear_status(dev)
+    else:
+        _status_host[_dev_index(dev)].zero_()
     return word
 
 
