@@ -622,12 +622,13 @@ def test_recorded_failure_is_raised_once_with_calls_in_flight(cuda):
     q, k, v = (t.to(cuda) for t in _qkv(1, 300, 300, 4, 2, 128, seed=13))
     good = T.attention(q, k, v)
     torch.cuda.synchronize(cuda)
+    torch.cuda._sleep(60_000_000)  # some 30 ms, in which all of this is queued
     ops._workspace(cuda)[:4].view(torch.int32).fill_(4)
     T.attention(q, k, v)
     seen = torch.cuda.Event()
     seen.record()
-    torch.cuda._sleep(40_000_000)  # some 20 ms
-    T.attention(q, k, v)           # queued behind it: reports once more
+    torch.cuda._sleep(60_000_000)
+    T.attention(q, k, v)           # reports once more, long after the first one
     seen.synchronize()
     with pytest.raises(T._lib.TrinixB200Error):
         T.attention(q, k, v)
