@@ -2,6 +2,7 @@
 attention), through triton_attn_func / the C ABI. Tolerance from the project baseline:
 2e-2 max abs error in bf16."""
 import ctypes
+import threading
 
 import pytest
 import torch
@@ -635,4 +636,57 @@ def test_recorded_failure_is_raised_once_with_calls_in_flight(cuda):
     for _ in range(3):
         assert torch.equal(T.attention(q, k, v), good)
         torch.cuda.synchronize(cuda)
+    assert T.attention_status(cuda) == 0
+
+
+@pytest.fixture
+def no_workspace_yet(cuda, monkeypatch):
+    """The state before a device's first attention call."""
+    from trinix_b200 import ops
+    T.attention(*(t.to(cuda) for t in _qkv(1, 16, 16, 2, 2, 64)))  # the library is loaded
+    torch.cuda.synchronize(cuda)
+    for name in ("_workspaces", "_status_host", "_status_word"):
+        monkeypatch.setattr(ops, name, {})
+    return ops
+
+
+def test_first_calls_from_several_threads_share_one_workspace(cuda, no_workspace_yet):
+    """One workspace and one host word per device, whoever comes first: a word that only a dropped
+    workspace still points at would be written after it was given back."""
+    ops, n = no_workspace_yet, 8
+    start, got = threading.Barrier(n), [None] * n
+
+    def first(i):
+        start.wait()
+        ws = ops._workspace(cuda)
+        got[i] = (ws.data_ptr(), ops._status_host[0].data_ptr(), ctypes.addressof(ops._status_word[0]))
+
+    threads = [threading.Thread(target=first, args=(i,)) for i in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(set(got)) == 1 and got[0][1] == got[0][2]
+    attached = int(ops._workspace(cuda)[8:16].view(torch.int64).item())
+    assert attached == got[0][1]  # unified addressing: the device's address of the word is the host's
+
+
+def test_new_workspace_is_ready_for_every_stream(cuda, no_workspace_yet):
+    side = torch.cuda.Stream(cuda)
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        ws = no_workspace_yet._workspace(cuda)
+    assert side.query()  # nothing of its set-up is still to run when another stream uses it
+    assert int(ws[:4].view(torch.int32).item()) == 0
+
+
+def test_first_call_under_capture(cuda, no_workspace_yet):
+    """The set-up is then part of the graph."""
+    q, k, v = (t.to(cuda) for t in _qkv(1, 200, 200, 4, 2, 128, seed=17))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = T.attention(q, k, v, causal=True)
+    graph.replay()
+    torch.cuda.synchronize(cuda)
+    assert torch.equal(out, T.attention(q, k, v, causal=True))
     assert T.attention_status(cuda) == 0

@@ -7,6 +7,7 @@ raise otherwise — there is no CPU path and no fallback.
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -488,6 +489,7 @@ def layernorm_backward(dy: torch.Tensor, x: torch.Tensor, weight: Optional[torch
 _workspaces: dict = {}
 _status_host: dict = {}  # device index -> pinned int32[1] mirror of the status word
 _status_word: dict = {}  # device index -> the mirror as a ctypes integer: read on every call
+_workspace_lock = threading.Lock()  # held by the thread that makes a device's three
 
 
 def _dev_index(dev: torch.device) -> int:
@@ -495,18 +497,32 @@ def _dev_index(dev: torch.device) -> int:
 
 
 def _workspace(dev: torch.device) -> torch.Tensor:
+    """The device's attention workspace: 256 zeroed bytes that every call on the device shares, with
+    a pinned host word attached that a failing launch writes. Whichever thread comes first makes
+    both; they are published when the set-up has run, so any thread and stream may use them (a first
+    call under stream capture, which cannot be waited for, makes the set-up part of its graph)."""
     idx = _dev_index(dev)
     ws = _workspaces.get(idx)
     if ws is None:
-        n = int(_lib.load().trx_attn_workspace_bytes())
+        with _workspace_lock:
+            ws = _workspaces.get(idx)
+            if ws is None:
+                ws = _make_workspace(idx)
+    return ws
+
+
+def _make_workspace(idx: int) -> torch.Tensor:
+    n = int(_lib.load().trx_attn_workspace_bytes())
+    host = torch.zeros(1, dtype=torch.int32).pin_memory()
+    with torch.cuda.device(idx):
         ws = torch.zeros(n, dtype=torch.uint8, device=torch.device("cuda", idx))
-        host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        with torch.cuda.device(idx):
-            _lib.check("trx_attn_mirror", _lib.load().trx_attn_mirror(
-                ws.data_ptr(), host.data_ptr(), _raw_stream(idx)))
-        _status_host[idx] = host
-        _status_word[idx] = ctypes.c_int32.from_address(host.data_ptr())
-        _workspaces[idx] = ws
+        _lib.check("trx_attn_mirror", _lib.load().trx_attn_mirror(
+            ws.data_ptr(), host.data_ptr(), _raw_stream(idx)))
+        if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(idx).synchronize()
+    _status_host[idx] = host
+    _status_word[idx] = ctypes.c_int32.from_address(host.data_ptr())
+    _workspaces[idx] = ws  # last: a thread that finds it finds the words too
     return ws
 
 
