@@ -508,6 +508,33 @@ def test_few_query_rows(cuda, Sq, Sk, Hq, Hk, D, causal, window, alibi, dtype):
     assert not out.float().cpu()[~rows].any()
 
 
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hk,D", [
+    (1, 16, 96, 32, 8, 128), (1, 16, 97, 32, 8, 128),      # the lines of the dispatch by keys
+    (1, 16, 128, 32, 8, 128), (1, 16, 129, 32, 8, 128),
+    (10, 16, 128, 32, 8, 128),     # more than one wave of the tcgen05 kernel
+    (24, 16, 256, 32, 8, 128),     # one CTA per row tile, two waves
+    (48, 1, 2093, 32, 8, 128),     # two, more than one wave
+    (8, 16, 1024, 32, 8, 128),     # two, one wave
+    (20, 1, 300, 8, 8, 64), (2, 2, 900, 32, 8, 128),       # one, four
+    (2, 1, 4093, 8, 8, 64), (3, 16, 5000, 8, 2, 128),      # eight
+    (1, 1, 9001, 8, 2, 64), (2, 3, 33000, 32, 1, 128),     # sixteen
+])
+def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
+    """Shapes for which the keys of a row tile go to 1, 2, 4, 8 and 16 CTAs, whatever the numbers the
+    cost arrives at. Reference in fp32 on the device; bounds as in test_few_query_rows."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(B, Sq, Sk, Hq, Hk, D, seed=Sk))
+    out, lse = ops.attention(q, k, v, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    qg = q.float().view(B, Sq, Hk, Hq // Hk, D)
+    s = torch.einsum("bihgd,bjhd->bhgij", qg, k.float()) * D ** -0.5
+    ref = torch.einsum("bhgij,bjhd->bihgd", torch.softmax(s, -1), v.float()).reshape(B, Sq, Hq, D)
+    assert float((out.float() - ref).abs().max()) <= TOL
+    ref_lse = torch.logsumexp(s, -1).reshape(B, Hq, Sq)
+    # sums of up to 33000 fp32 terms in another order: below 33000 * 2^-24 of the sum
+    assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
+
+
 @pytest.mark.parametrize("Sq", [1, 4])
 def test_few_query_rows_in_every_layout(cuda, Sq):
     """The same call with contiguous tensors, transposed (B, H, S, D) storage, a slice of a longer

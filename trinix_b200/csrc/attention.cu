@@ -21,7 +21,8 @@
 // h / (Hq / Hk), so GQA / MQA need no tiled copies. With ALiBi under a causal mask the KV tiles
 // of a row block are visited from the diagonal backwards: the bias grows with the key index, so
 // in that order the first tile holds the row maximum and O is never rescaled again.
-// Calls of up to 16 query rows without mask or dropout take the kernel of attention_decode.cuh.
+// Calls of up to 16 query rows without mask or dropout take the kernel of attention_decode.cuh (but
+// for a few, see use_decode).
 //
 // Every wait on an mbarrier is bounded: after a fixed number of polls the kernel records a
 // code in the status word of the caller's workspace, raises a CTA-wide abort flag, drains its
@@ -1313,7 +1314,13 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   p.k_hdiv = k_hb ? static_cast<int>(Hq) : group;
   p.v_hdiv = v_hb ? static_cast<int>(Hq) : group;
   p.group = p.k_hdiv < p.v_hdiv ? p.k_hdiv : p.v_hdiv;
-  p.decode = !bias && dropout_p == 0.0f && use_decode(Sq, Hq, p.group) ? 1 : 0;
+  p.B = static_cast<int>(B);
+  p.Sq = static_cast<int>(Sq);
+  p.Sk = static_cast<int>(Sk);
+  p.Hq = static_cast<int>(Hq);
+  // two query heads per CTA when each pair (2i, 2i + 1) reads one kv head in K and in V
+  p.pair_heads = (Hq % 2 == 0 && p.k_hdiv % 2 == 0 && p.v_hdiv % 2 == 0) ? 1 : 0;
+  p.decode = !bias && dropout_p == 0.0f && use_decode(p, D) ? 1 : 0;
   const int kv_box = p.decode ? DEC_KEYS : ATT_BN;
   rc = make_map(&p.tm_k, kk, is_bf16, D, Sk_map, k_hb ? 1 : Hk, k_bb ? 1 : B, k_strides[0],
                 k_strides[1], k_strides[2], kv_box);
@@ -1325,10 +1332,6 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   p.lse = lse_or_null;
   p.slopes = slopes_or_null;
   p.status = reinterpret_cast<unsigned int*>(workspace);
-  p.B = static_cast<int>(B);
-  p.Sq = static_cast<int>(Sq);
-  p.Sk = static_cast<int>(Sk);
-  p.Hq = static_cast<int>(Hq);
   p.q = q;
   p.q_stride_b = q_strides[0];
   p.q_stride_s = q_strides[1];
@@ -1351,8 +1354,6 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   // with it comes a rescale of the whole O accumulator; walking them backwards the first tile
   // holds the maximum and later ones never beat it by more than the lazy-rescale margin.
   p.reverse_kv = (slopes_or_null != nullptr && (causal || window_right == 0)) ? 1 : 0;
-  // two query heads per CTA when each pair (2i, 2i + 1) reads one kv head in K and in V
-  p.pair_heads = (Hq % 2 == 0 && p.k_hdiv % 2 == 0 && p.v_hdiv % 2 == 0) ? 1 : 0;
   if (bias && Sk > 0) {
     p.bias = bias;
     p.bias_sb = bias_strides[0];

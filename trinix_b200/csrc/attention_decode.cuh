@@ -8,13 +8,16 @@
 // sequences of 4093 keys (32 / 8 heads, head dim 128), 1.9 TB/s; one sequence of 32768 keys
 // 507 us. Here (45.0 us, 6.0 TB/s; 34.6 us)
 //   * the query heads of a kv head and their rows are packed into tiles of 16 rows, the M of one
-//     mma.sync.m16n8k16: nothing is read twice, and the padding is 16 rows and not 128;
+//     mma.sync.m16n8k16, one or two tiles to a warp: K and V are read once per 16 or 32 packed rows,
+//     i.e. once for up to 32 of them (again for more, mostly from L2), and the padding is less than
+//     one such tile and not 128 rows;
 //   * the keys are split over the CTAs of a thread-block cluster and, inside a CTA, over its four
 //     warps. Each warp owns a ring of 16-key K and V tiles (TMA, 128-byte swizzle, its own
 //     mbarriers) and its own running maximum, sum and O accumulators, so no warp waits for
 //     another one before the end;
 //   * the partial results meet in shared memory, then over distributed shared memory inside the
-//     cluster: no workspace, one launch, a fixed order of the sums.
+//     cluster: no workspace, one launch, and sums in an order fixed by the shape of the whole call
+//     (the number of splits goes by the batch, too) and the SM count of the device.
 // Scores, sums and O are fp32, probabilities go into the second product in the activation dtype,
 // as in the tcgen05 kernel; an mma.sync at M = 16 is issued 32 times per 8 KB of keys, so the
 // tensor pipe idles beside the memory system either way.
@@ -399,26 +402,38 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM)
   cluster.sync();  // no CTA leaves while another one reads its shared memory
 }
 
-// CTAs that share the keys of one row tile: as many as still find room on the chip at once while
-// every warp keeps two tiles; two where that shortens a launch of more CTAs than there is room for
-// (ceil(units * 2 / slots) / 2 waves against ceil(units / slots)). More and larger clusters lose:
-// their CTAs need room in one GPC at the same time. Measured, 32 / 8 heads, head dim 128:
-// 6 x 8000 keys (48 units) 35.1 us with 4 CTAs per unit, 54.8 us with 16; 20 x 4093 keys (160
-// units) 60.0 us with one, 67.9 us with 8; 48 x 2093 keys (384 units) 76.6 us with one, 70.9 us
-// with two.
-static int decode_splits(const AttnParams& p, int64_t units) {
+// CTAs that share the keys of one row tile: the power of two that a cost, in quarters of the time
+// of one 16-key tile (0.75 to 1.1 us), makes the cheapest. A CTA costs a start and an end (14), the merge of a
+// cluster 10 more; a second CTA on an SM slows both down at either end (5, with two row tiles per
+// warp 10); clusters of 8 and 16 wait for room in one GPC once there are many of them. Fitted to
+// every split of 2624 shapes (1 to 16 rows, 64 to 32768 keys, 1 to 1536 units, both head dims): 1.7 %
+// slower than the best split in the mean. Splitting wherever a warp keeps two tiles and the chip has
+// room, and by two for every last wave that is under half full, is 6.0 % slower, and far off in
+// single shapes (32 / 8 heads, head dim 128, that / this / the tcgen05 kernel): 24 x 256 keys, 16 rows
+// 40.6 / 23.7 / 28.6 us; 8 x 256 keys, 16 rows 14.8 / 11.2 / 10.8 us; 2 x 4096 keys, 1 row 18.2 / 12.6
+// / 69.5 us.
+static int decode_splits(const AttnParams& p, int64_t units, bool wide) {
   int64_t keys = p.Sk;  // that some row sees
   if (p.causal && p.Sq < keys) keys = p.Sq;
   if (p.win_right >= 0 && static_cast<int64_t>(p.Sq) + p.win_right < keys) keys = p.Sq + p.win_right;
   if (p.win_left >= 0 && static_cast<int64_t>(p.Sq) + p.win_left + p.win_right < keys)
     keys = p.Sq + p.win_left + p.win_right;
-  const int64_t slots = static_cast<int64_t>(sm_count_of_current_device()) * DEC_CTAS_PER_SM;
+  const int64_t sms = sm_count_of_current_device(), slots = sms * DEC_CTAS_PER_SM;
   const int64_t tiles = (keys + DEC_KEYS - 1) / DEC_KEYS;
-  int n = 1;
-  while (n < DEC_MAX_SPLIT && units * n * 2 <= slots && tiles >= n * 4 * DEC_WARPS) n *= 2;
-  const int64_t whole = (units + slots - 1) / slots, halved = (units * 2 + slots - 1) / slots;
-  if (n == 1 && halved < 2 * whole && whole > 1 && tiles >= 4 * DEC_WARPS) n = 2;
-  return n;
+  auto cost = [&](int64_t n) {
+    const int64_t ctas = units * n, waves = (ctas + slots - 1) / slots;
+    const int64_t chain = (tiles + n * DEC_WARPS - 1) / (n * DEC_WARPS);
+    int64_t ends = 14;
+    if (n > 1) ends += waves > 1 ? 13 : 10;
+    if (ctas > sms) ends += wide ? 10 : 5;
+    if (n >= 8 && ctas > 64) ends += n == 8 ? 4 : 6;
+    if (n == 16) ends += 1;
+    return waves * (ends + 4 * chain);
+  };
+  int best = 1;
+  for (int n = 2; n <= DEC_MAX_SPLIT && tiles >= n * DEC_WARPS; n *= 2)
+    if ((n == 2 || units * n <= slots) && cost(n) < cost(best)) best = n;
+  return best;
 }
 
 template <int D, bool BF16, int MT>
@@ -441,7 +456,7 @@ static int launch_decode(const AttnParams& p, cudaStream_t stream) {
                         ((static_cast<int64_t>(p.group) * p.Sq + L::ROWS - 1) / L::ROWS);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr{};
-  const unsigned n = static_cast<unsigned>(decode_splits(p, units * p.B));
+  const unsigned n = static_cast<unsigned>(decode_splits(p, units * p.B, MT == 2));
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = n;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
@@ -457,10 +472,15 @@ static int launch_decode(const AttnParams& p, cudaStream_t stream) {
 // Calls that take this kernel: up to 16 query rows. The tcgen05 kernel spends the same time on any
 // Sq up to 128 (it works on whole 128-row tiles), this one works on tiles of 16 packed rows.
 // Measured at 4096 keys, head dim 128, this / the tcgen05 kernel: Sq = 16, B = 16, 32 / 32 heads
-// 159 / 269 us; 32 / 8 heads 91 / 140 us; Sq = 64, B = 4, 32 / 8 heads 90 / 71 us.
-static bool use_decode(int64_t Sq, int64_t Hq, int64_t group) {
-  const int64_t rows = Sq * group;
-  return Sq <= 16 && (Hq / group) * ((rows + 15) / 16) <= 65535;
+// 159 / 269 us; 32 / 8 heads 91 / 140 us; 32 / 1 heads (512 packed rows) 88 / 139 us, B = 1 29 / 69
+// us; Sq = 64, B = 4, 32 / 8 heads 90 / 71 us. The exception is a single key tile of the tcgen05 kernel
+// that is nearly full, in one wave of CTAs, at head dim 128, against two row tiles per warp here: 97
+// to 128 keys 8.4 to 8.8 / 7.6 to 8.2 us whatever the batch (96 keys 8.3 / 8.2; 129 keys 9.1 / 10.6).
+static bool use_decode(const AttnParams& p, int64_t D) {
+  const int64_t rows = static_cast<int64_t>(p.Sq) * p.group;
+  if (p.Sq > 16 || (p.Hq / p.group) * ((rows + 15) / 16) > 65535) return false;
+  const int64_t ctas = static_cast<int64_t>(p.B) * (p.pair_heads ? p.Hq / 2 : p.Hq);
+  return !(D == 128 && rows > 16 && p.Sk > 96 && p.Sk <= ATT_BN && ctas <= sm_count_of_current_device());
 }
 
 }  // namespace trx
