@@ -338,8 +338,8 @@ def test_empty_and_invalid_backward_inputs(cuda):
 @pytest.mark.parametrize("rows,cols", [(1, 8), (7, 1000), (64, 4096), (3, 4104), (2, 16384), (3, 777)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_norm_backward_with_the_forwards_statistics(cuda, rows, cols, dtype):
-    """The forward's rstd (and mean) against recomputed ones, in every width class and on the scalar
-    path, with and without a residual. The statistics differ in their last fp32 bits only (sums in
+    """The forward's rstd (and mean) against recomputed ones, in rows of 1 to 2052 vectors and on the
+    scalar path, with and without a residual (every width class: the walk over several rows, below). The statistics differ in their last fp32 bits only (sums in
     another order, 2^-22 relative), so the fp32 gradients differ by a few times that and 16-bit ones
     by at most one rounding (2^-8 / 2^-11 of the value, twice half an ulp)."""
     g = torch.Generator().manual_seed(rows + cols)
@@ -373,7 +373,7 @@ def test_norm_backward_with_the_forwards_statistics(cuda, rows, cols, dtype):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_norm_backward_at_the_edges_of_the_width_classes(cuda, nvec, dtype):
     """Rows of the widest and narrowest width of every launch configuration (and the first one on
-    the scalar path), more rows than one CTA walks in some, statistics recomputed and saved: against
+    the scalar path), one row per CTA, statistics recomputed and saved: against
     the float64 oracle within the bounds of the shape test (dx: one output rounding; dW and db: an
     fp32 sum over the rows, then one rounding)."""
     cols = nvec * (4 if dtype == torch.float32 else 8)
@@ -393,3 +393,51 @@ def test_norm_backward_at_the_edges_of_the_width_classes(cuda, nvec, dtype):
         dx, dw, db = T.ops.layernorm_backward(dyc, xc, wc, 1e-5, **kw_l)
         assert rel_err(dx.cpu().double(), lx) <= tol and rel_err(dw.cpu().double(), lw) <= tol_sum
         assert rel_err(db.cpu().double(), lb) <= tol_sum
+
+
+@pytest.mark.parametrize("nvec", [40, 100, 200, 300, 600, 900, 1030, 2048])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_norm_backward_over_several_rows_per_cta(cuda, nvec, dtype):
+    """One width of every class, few enough rows for the configurations that few rows take and more
+    than any grid has CTAs (three per SM for narrow rows, fewer for wide ones), so that every CTA
+    walks several rows: running column sums, prefetched rows, alternating reduction banks.
+    RMSNorm, its activation form and LayerNorm, with and without a residual, statistics recomputed
+    and saved, against float64 autograd on the device. Bounds relative to |value| + rms: a dx is a
+    difference of terms of the size of the rms with some 8 fp32 roundings each (mish' has the most),
+    8 * 2^-24 = 5e-7 of up to 5 rms; a dw is a sum in which every partial sum takes part in at most 17
+    (rows of a CTA) + 14 + 32 (partial rows) additions, 63 * 2^-24 = 4e-6 of it; so 5e-6, and for
+    16-bit results one rounding more (half an ulp: 2^-9, 2^-12)."""
+    cols = nvec * (4 if dtype == torch.float32 else 8)
+    tol = {torch.float32: 5e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    for rows in (7 * sms // 2, 17 * sms) if nvec <= 1024 else (7 * sms // 2,):
+        g = torch.Generator(device=cuda).manual_seed(nvec + rows)
+        x, r, dy = (torch.randn(rows, cols, generator=g, device=cuda).to(dtype) for _ in range(3))
+        w, b = (torch.randn(cols, generator=g, device=cuda).to(dtype) for _ in range(2))
+
+        def exact(res, ln, act):
+            xd = (x.double() + res.double() if res is not None else x.double()).requires_grad_(True)
+            wd = w.double().requires_grad_(True)
+            d = xd - xd.mean(-1, keepdim=True) if ln else xd
+            y = d * torch.rsqrt(d.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+            if act:
+                y = y * torch.tanh(torch.nn.functional.softplus(y))
+            return torch.autograd.grad(y, (xd, wd), dy.double())
+
+        def check(got, res, ln=False, act=False):
+            for a, b in zip(got, (*exact(res, ln, act), dy.double().sum(0))):
+                assert a.dtype == dtype and a.shape == b.shape
+                assert bool(((a.double() - b).abs() <= tol * (b.abs() + b.pow(2).mean().sqrt())).all())
+
+        for res in (None, r):
+            if res is None:
+                _, rstd = T.ops.rmsnorm(x, w, 1e-6, return_rstd=True)
+                _, mean, ln_rstd = T.ops.layernorm(x, w, b, 1e-6, return_stats=True)
+                check(T.ops.rmsnorm_backward(dy, x, w, 1e-6, activation="mish"), None, act=True)
+            else:
+                _, rstd = T.ops.residual_rmsnorm(x, res, w, 1e-6, return_rstd=True)
+                _, mean, ln_rstd = T.ops.residual_layernorm(x, res, w, b, 1e-6, return_stats=True)
+            for saved in ({}, {"rstd": rstd}):
+                check(T.ops.rmsnorm_backward(dy, x, w, 1e-6, residual=res, **saved), res)
+            for saved in ({}, {"mean": mean, "rstd": ln_rstd}):
+                check(T.ops.layernorm_backward(dy, x, w, 1e-6, residual=res, **saved), res, ln=True)

@@ -2,7 +2,7 @@
 //
 // Norms. A CTA of 64 to 512 threads walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; a row of x and
 // of dy is read from HBM once with 128-bit streaming loads and stays in registers. The row's
-// statistics are the forward's (SAVED) or recomputed from x; what bounds the kernel is the latency
+// statistics are the forward's or recomputed from x; what bounds the kernel is the latency
 // of the CTA-wide reductions of a row at 12 to 24 warps per SM, and the saved statistics leave one
 // of three (LayerNorm, 32768 x 4096 bf16: 166.4 -> 151.5 us) or of two (RMSNorm: 149.6 -> 136.4
 // us). dx is written, and every thread keeps fp32 running sums of dy * n (and dy) for the columns it owns. At the end
@@ -30,6 +30,10 @@
 
 namespace trx {
 
+// Within 128 bytes: past that the compiler reads the fields where they are used instead of holding
+// them, and a row loop tests `res` and `act` vector by vector (16384 x 4096 bf16 at 144 bytes / here:
+// RMSNorm 79.6 / 77.2 us, its activation form 144.6 / 138.5, with a residual 105.7 / 95.1, LayerNorm
+// with a residual 136.3 / 109.2, the same with the forward's statistics 124.8 / 102.3).
 struct NormBwdParams {
   const void* dy;
   const void* x;
@@ -40,13 +44,19 @@ struct NormBwdParams {
   float* db_part;    // (P, C) fp32 or null
   const float* mean;  // (R) row statistics as the forward had them, or null: recomputed from x
   const float* rstd;
-  float* stats;      // (R, 2) fp32: mean, rstd (scalar path only)
   int64_t R, C;
   int64_t dy_stride, x_stride, dx_stride, res_stride;  // elements
   float eps;
-  int w_dtype;
-  int act;           // -1: plain norm; TRX_ACT_*: the upstream gradient is dy * act'(w * n)
+  signed char w_dtype;
+  signed char act;   // -1: plain norm; TRX_ACT_*: the upstream gradient is dy * act'(w * n)
 };
+static_assert(sizeof(NormBwdParams) <= 128, "see above");
+
+// Row statistics of the vector kernel: recomputed from the row, or the forward's. RMSNorm with the
+// forward's statistics knows at compile time whether its rows are sums x + res (8192 x 8192 bf16
+// without one 80.4 us at run time, 75.3 here; 10922 x 1536 fp32 with one 52.7 / 48.1); recomputing
+// kernels and LayerNorm gain nothing from that or lose (131072 x 512 bf16 LayerNorm 135.8 / 161.6).
+enum NormStats { STATS_RECOMPUTED, STATS_SAVED, STATS_SAVED_OF_SUM };
 
 // Sum of a float2 over the NT threads of a CTA; two alternating banks, one barrier.
 template <int NT = 256>
@@ -111,7 +121,7 @@ __device__ __forceinline__ float act_grad(int act, float z) {
 
 // MIN_CTAS: resident CTAs per SM asked of the compiler (caps the registers per thread; without it
 // the compiler spends them freely and the occupancy drops).
-template <bool LN, bool SAVED, typename T, int VPT, int NT, int MIN_CTAS>
+template <bool LN, NormStats STATS, typename T, int VPT, int NT, int MIN_CTAS>
 __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdParams p) {
   using P = Pack<T>;
   constexpr int VEC = P::VEC;
@@ -122,6 +132,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
   const float inv_C = __fdiv_rn(1.0f, static_cast<float>(p.C));
 
   constexpr int H2 = VEC / 2;
+  const bool has_res = LN || STATS == STATS_RECOMPUTED ? p.res != nullptr : STATS == STATS_SAVED_OF_SUM;
   float2 dwacc[VPT][H2];
   float2 dbacc[LN ? VPT : 1][H2];
 #pragma unroll
@@ -136,7 +147,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
     const T* xrow = reinterpret_cast<const T*>(p.x) + row * p.x_stride;
     const T* grow = reinterpret_cast<const T*>(p.dy) + row * p.dy_stride;
     float mean = 0.0f, rstd = 0.0f;
-    if constexpr (SAVED) {
+    if constexpr (STATS != STATS_RECOMPUTED) {
       if constexpr (LN) mean = __ldg(p.mean + row);
       rstd = __ldg(p.rstd + row);
     }
@@ -155,7 +166,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
         const uint32_t row_bytes = static_cast<uint32_t>(nvec) * 16u;
         l2_prefetch_bulk(reinterpret_cast<const T*>(p.x) + prow * p.x_stride, row_bytes);
         l2_prefetch_bulk(reinterpret_cast<const T*>(p.dy) + prow * p.dy_stride, row_bytes);
-        if (p.res) l2_prefetch_bulk(reinterpret_cast<const T*>(p.res) + prow * p.res_stride, row_bytes);
+        if (has_res) l2_prefetch_bulk(reinterpret_cast<const T*>(p.res) + prow * p.res_stride, row_bytes);
       }
     }
     // fp32 pairs: the arithmetic below is packed (two lanes per instruction)
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
       P::unpack2(xr[i], xf[i]);
       P::unpack2(gr[i], gf[i]);
     }
-    if (p.res) {  // residual forms: the normalised row is the fp32 sum x + r, as in the forward
+    if (has_res) {  // residual forms: the normalised row is the fp32 sum x + r, as in the forward
       const T* rrow = reinterpret_cast<const T*>(p.res) + row * p.res_stride;
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
@@ -179,7 +190,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
       }
     }
     // ---- statistics: the forward's, or recomputed from x ----------------------------
-    if constexpr (SAVED) {
+    if constexpr (STATS != STATS_RECOMPUTED) {
       if constexpr (LN) {
         const float2 nmean2 = make_float2(-mean, -mean);
 #pragma unroll
@@ -293,9 +304,10 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
   }
 }
 
-// Scalar path, step 1: dx for any C and alignment, (mean, rstd) of every row into p.stats.
+// Scalar path, step 1: dx for any C and alignment, (mean, rstd) of every row into stats (R, 2).
 template <bool LN, typename T>
-__global__ void __launch_bounds__(256) norm_bwd_generic_dx(const NormBwdParams p) {
+__global__ void __launch_bounds__(256) norm_bwd_generic_dx(const NormBwdParams p,
+                                                           float* stats) {
   using P = Pack<T>;
   __shared__ float2 red[2][8];
   int sel = 0;
@@ -349,16 +361,17 @@ __global__ void __launch_bounds__(256) norm_bwd_generic_dx(const NormBwdParams p
       }
       P::store1(dxrow + c, rstd * (g - c2 - n * c1));
     }
-    if (threadIdx.x == 0 && p.stats) {
-      p.stats[2 * row] = mean;
-      p.stats[2 * row + 1] = rstd;
+    if (threadIdx.x == 0) {
+      stats[2 * row] = mean;
+      stats[2 * row + 1] = rstd;
     }
   }
 }
 
 // Scalar path, step 2: one thread per column, one row slice per blockIdx.y.
 template <typename T>
-__global__ void __launch_bounds__(256) norm_bwd_generic_partials(const NormBwdParams p) {
+__global__ void __launch_bounds__(256) norm_bwd_generic_partials(const NormBwdParams p,
+                                                                 const float* stats) {
   using P = Pack<T>;
   const int64_t c = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (c >= p.C) return;
@@ -367,7 +380,7 @@ __global__ void __launch_bounds__(256) norm_bwd_generic_partials(const NormBwdPa
     const float dyv = P::load1(reinterpret_cast<const T*>(p.dy) + row * p.dy_stride + c);
     float xv = P::load1(reinterpret_cast<const T*>(p.x) + row * p.x_stride + c);
     if (p.res) xv += P::load1(reinterpret_cast<const T*>(p.res) + row * p.res_stride + c);
-    const float n = (xv - p.stats[2 * row]) * p.stats[2 * row + 1];
+    const float n = (xv - stats[2 * row]) * stats[2 * row + 1];
     float dz = dyv;
     if (p.act >= 0) dz *= act_grad<sizeof(T) == 2>(p.act, n * load_param1(p.w, p.w_dtype, c));
     dw = fmaf(dz, n, dw);
@@ -423,7 +436,7 @@ static int64_t norm_bwd_partial_rows(int64_t R, int64_t C) {
 
 // TRX_BWD_WAVES resident waves of CTAs (each walks R / grid rows); P_rows comes back as the grid size, i.e.
 // the number of rows of partial sums that were written.
-template <bool LN, bool SAVED, typename T, int VPT, int NT, int MIN_CTAS>
+template <bool LN, NormStats STATS, typename T, int VPT, int NT, int MIN_CTAS>
 static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStream_t stream) {
   static std::atomic<int> blocks_per_sm_of[64];  // racing first calls store the same value
   int dev = 0;
@@ -432,7 +445,7 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   int blocks_per_sm = cacheable ? blocks_per_sm_of[dev].load(std::memory_order_acquire) : 0;
   if (blocks_per_sm == 0) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, SAVED, T, VPT, NT, MIN_CTAS>, NT, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_bwd_kernel<LN, STATS, T, VPT, NT, MIN_CTAS>, NT, 0) !=
             cudaSuccess || n <= 0)
       n = 1;
     blocks_per_sm = n;
@@ -440,10 +453,10 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
   }
   const int64_t resident = static_cast<int64_t>(sm_count_of_current_device()) * blocks_per_sm * TRX_BWD_WAVES;
   if (P_rows > resident) P_rows = resident;
-  norm_bwd_kernel<LN, SAVED, T, VPT, NT, MIN_CTAS><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
+  norm_bwd_kernel<LN, STATS, T, VPT, NT, MIN_CTAS><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
 }
 
-template <bool LN, bool SAVED, typename T>
+template <bool LN, NormStats STATS, typename T>
 static void launch_norm_bwd_width(const NormBwdParams& p, int64_t nvec, int64_t& P_rows,
                                   cudaStream_t stream) {
   // A row's threads meet in CTA-wide reductions, so few warps per row and many CTAs per SM are what
@@ -462,16 +475,16 @@ static void launch_norm_bwd_width(const NormBwdParams& p, int64_t nvec, int64_t&
   //   8192 x 5120 fp32          107.2 / 104.4               125.0 / 117.5              387 / 356
   constexpr bool F32 = Pack<T>::VEC == 4;
   constexpr int V256 = LN || !F32 ? 2 : 1;
-  if (nvec <= 64) launch_norm_bwd_vec<LN, SAVED, T, 1, 64, 12>(p, P_rows, stream);
-  else if (nvec <= 128) launch_norm_bwd_vec<LN, SAVED, T, 1, 128, 6>(p, P_rows, stream);
-  else if (nvec <= 256) launch_norm_bwd_vec<LN, SAVED, T, V256, 256 / V256, V256 == 2 ? 5 : 3>(p, P_rows, stream);
-  else if (nvec <= 512) launch_norm_bwd_vec<LN, SAVED, T, LN ? 4 : 2, LN ? 128 : 256, 3>(p, P_rows, stream);
-  else if (nvec <= 768) launch_norm_bwd_vec<LN, SAVED, T, 3, 256, 2>(p, P_rows, stream);
+  if (nvec <= 64) launch_norm_bwd_vec<LN, STATS, T, 1, 64, 12>(p, P_rows, stream);
+  else if (nvec <= 128) launch_norm_bwd_vec<LN, STATS, T, 1, 128, 6>(p, P_rows, stream);
+  else if (nvec <= 256) launch_norm_bwd_vec<LN, STATS, T, V256, 256 / V256, V256 == 2 ? 5 : 3>(p, P_rows, stream);
+  else if (nvec <= 512) launch_norm_bwd_vec<LN, STATS, T, LN ? 4 : 2, LN ? 128 : 256, 3>(p, P_rows, stream);
+  else if (nvec <= 768) launch_norm_bwd_vec<LN, STATS, T, 3, 256, 2>(p, P_rows, stream);
   else if (nvec <= 1024) {
-    if constexpr (LN && !F32) launch_norm_bwd_vec<LN, SAVED, T, 2, 512, 1>(p, P_rows, stream);
-    else launch_norm_bwd_vec<LN, SAVED, T, 4, 256, 2>(p, P_rows, stream);
+    if constexpr (LN && !F32) launch_norm_bwd_vec<LN, STATS, T, 2, 512, 1>(p, P_rows, stream);
+    else launch_norm_bwd_vec<LN, STATS, T, 4, 256, 2>(p, P_rows, stream);
   } else {
-    launch_norm_bwd_vec<LN, SAVED, T, 4, 512, 1>(p, P_rows, stream);
+    launch_norm_bwd_vec<LN, STATS, T, 4, 512, 1>(p, P_rows, stream);
   }
 }
 
@@ -481,7 +494,7 @@ static int launch_norm_bwd(NormBwdParams p, void* dw, void* db, float* ws, cudaS
   int64_t P_rows = norm_bwd_partial_rows(p.R, p.C);
   float* part0 = ws;
   float* part1 = ws + norm_bwd_partial_rows(p.R, p.C) * p.C;
-  p.stats = part1 + norm_bwd_partial_rows(p.R, p.C) * p.C;
+  float* stats = part1 + norm_bwd_partial_rows(p.R, p.C) * p.C;
   p.dw_part = dw ? part0 : nullptr;
   p.db_part = db ? part1 : nullptr;
   if (p.R > 0) {
@@ -492,14 +505,15 @@ static int launch_norm_bwd(NormBwdParams p, void* dw, void* db, float* ws, cudaS
     if (p.res) vec_ok = vec_ok && aligned_to(p.res, 16) && (p.res_stride % VEC == 0);
     const int64_t nvec = p.C / VEC;
     if (vec_ok && nvec <= 2048) {
-      if (p.rstd) launch_norm_bwd_width<LN, true, T>(p, nvec, P_rows, stream);
-      else launch_norm_bwd_width<LN, false, T>(p, nvec, P_rows, stream);
+      if (!p.rstd) launch_norm_bwd_width<LN, STATS_RECOMPUTED, T>(p, nvec, P_rows, stream);
+      else if (LN || !p.res) launch_norm_bwd_width<LN, STATS_SAVED, T>(p, nvec, P_rows, stream);
+      else if constexpr (!LN) launch_norm_bwd_width<LN, STATS_SAVED_OF_SUM, T>(p, nvec, P_rows, stream);
     } else {
       const int64_t cap = static_cast<int64_t>(sm_count_of_current_device()) * 8;
-      norm_bwd_generic_dx<LN, T><<<static_cast<unsigned>(p.R < cap ? p.R : cap), 256, 0, stream>>>(p);
+      norm_bwd_generic_dx<LN, T><<<static_cast<unsigned>(p.R < cap ? p.R : cap), 256, 0, stream>>>(p, stats);
       if (dw || db) {
         const dim3 grid(static_cast<unsigned>((p.C + 255) / 256), static_cast<unsigned>(P_rows));
-        norm_bwd_generic_partials<T><<<grid, 256, 0, stream>>>(p);
+        norm_bwd_generic_partials<T><<<grid, 256, 0, stream>>>(p, stats);
       }
     }
   } else {
@@ -543,7 +557,9 @@ static int norm_bwd_entry(const void* dy, const void* x, const void* w, void* dx
   NormBwdParams p{};
   p.dy = dy; p.x = x; p.w = w; p.dx = dx; p.res = res; p.res_stride = res_stride;
   p.R = R; p.C = C; p.dy_stride = dy_stride; p.x_stride = x_stride; p.dx_stride = dx_stride;
-  p.eps = eps; p.w_dtype = w_dtype; p.act = act; p.mean = mean; p.rstd = rstd;
+  p.eps = eps; p.mean = mean; p.rstd = rstd;
+  p.w_dtype = static_cast<signed char>(w_dtype);
+  p.act = static_cast<signed char>(act);
   float* ws = static_cast<float*>(workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (x_dtype) {
