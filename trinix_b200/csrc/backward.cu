@@ -54,8 +54,10 @@ static_assert(sizeof(NormBwdParams) <= 128, "see above");
 
 // Row statistics of the vector kernel: recomputed from the row, or the forward's. RMSNorm with the
 // forward's statistics knows at compile time whether its rows are sums x + res (8192 x 8192 bf16
-// without one 80.4 us at run time, 75.3 here; 10922 x 1536 fp32 with one 52.7 / 48.1); recomputing
-// kernels and LayerNorm gain nothing from that or lose (131072 x 512 bf16 LayerNorm 135.8 / 161.6).
+// without one 80.4 us at run time, 75.3 here; 10922 x 1536 fp32 with one 52.7 / 48.1), and so does
+// LayerNorm in its widest class, which spills (5461 x 12288 bf16 without one 151.2 / 145.6, with one
+// 174.7 / 159.4). Recomputing kernels and narrower LayerNorms gain nothing from it or lose
+// (131072 x 512 bf16 LayerNorm 135.8 / 161.6).
 enum NormStats { STATS_RECOMPUTED, STATS_SAVED, STATS_SAVED_OF_SUM };
 
 // Sum of a float2 over the NT threads of a CTA; two alternating banks, one barrier.
@@ -132,7 +134,8 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) norm_bwd_kernel(const NormBwdPar
   const float inv_C = __fdiv_rn(1.0f, static_cast<float>(p.C));
 
   constexpr int H2 = VEC / 2;
-  const bool has_res = LN || STATS == STATS_RECOMPUTED ? p.res != nullptr : STATS == STATS_SAVED_OF_SUM;
+  constexpr bool KNOWS_RES = STATS != STATS_RECOMPUTED && (!LN || VPT * NT > 1024);
+  const bool has_res = KNOWS_RES ? STATS == STATS_SAVED_OF_SUM : p.res != nullptr;
   float2 dwacc[VPT][H2];
   float2 dbacc[LN ? VPT : 1][H2];
 #pragma unroll
@@ -506,8 +509,9 @@ static int launch_norm_bwd(NormBwdParams p, void* dw, void* db, float* ws, cudaS
     const int64_t nvec = p.C / VEC;
     if (vec_ok && nvec <= 2048) {
       if (!p.rstd) launch_norm_bwd_width<LN, STATS_RECOMPUTED, T>(p, nvec, P_rows, stream);
-      else if (LN || !p.res) launch_norm_bwd_width<LN, STATS_SAVED, T>(p, nvec, P_rows, stream);
-      else if constexpr (!LN) launch_norm_bwd_width<LN, STATS_SAVED_OF_SUM, T>(p, nvec, P_rows, stream);
+      else if (!p.res || (LN && nvec <= 1024)) launch_norm_bwd_width<LN, STATS_SAVED, T>(p, nvec, P_rows, stream);
+      else if constexpr (LN) launch_norm_bwd_vec<LN, STATS_SAVED_OF_SUM, T, 4, 512, 1>(p, P_rows, stream);
+      else launch_norm_bwd_width<LN, STATS_SAVED_OF_SUM, T>(p, nvec, P_rows, stream);
     } else {
       const int64_t cap = static_cast<int64_t>(sm_count_of_current_device()) * 8;
       norm_bwd_generic_dx<LN, T><<<static_cast<unsigned>(p.R < cap ? p.R : cap), 256, 0, stream>>>(p, stats);
