@@ -410,7 +410,7 @@ def test_norm_backward_over_several_rows_per_cta(cuda, nvec, dtype):
     cols = nvec * (4 if dtype == torch.float32 else 8)
     tol = {torch.float32: 5e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
     sms = torch.cuda.get_device_properties(cuda).multi_processor_count
-    for rows in (7 * sms // 2, 17 * sms) if nvec <= 1024 else (7 * sms // 2,):
+    for rows in (2 * sms, 7 * sms // 2, 17 * sms) if nvec <= 1024 else (7 * sms // 2,):
         g = torch.Generator(device=cuda).manual_seed(nvec + rows)
         x, r, dy = (torch.randn(rows, cols, generator=g, device=cuda).to(dtype) for _ in range(3))
         w, b = (torch.randn(cols, generator=g, device=cuda).to(dtype) for _ in range(2))

@@ -454,8 +454,20 @@ static void launch_norm_bwd_vec(const NormBwdParams& p, int64_t& P_rows, cudaStr
     blocks_per_sm = n;
     if (cacheable) blocks_per_sm_of[dev].store(n, std::memory_order_release);
   }
-  const int64_t resident = static_cast<int64_t>(sm_count_of_current_device()) * blocks_per_sm * TRX_BWD_WAVES;
+  const int64_t sms = sm_count_of_current_device();
+  const int64_t resident = sms * blocks_per_sm * TRX_BWD_WAVES;
   if (P_rows > resident) P_rows = resident;
+  // Each CTA leaves a row of partial sums, and adding them up is the longer half of a call with few
+  // rows (1024 x 1024 bf16 RMSNorm: dx 3.7 us, the sum of 1024 partial rows 6.6 us, of 444 4.1). So
+  // more than three CTAs per SM only where each gets four rows or more (that call 10.1 -> 8.2 us,
+  // 2048 x 512 9.8 -> 8.8), and for LayerNorm's two sums one per SM where that makes no more than
+  // two rows (204 x 5120 bf16 13.3 -> 12.1 us; RMSNorm's one sum gains nothing by it, 9.1 / 9.1).
+  if (MIN_CTAS > 3) {
+    const int64_t limit = p.R / 4 > 3 * sms ? p.R / 4 : 3 * sms;
+    if (P_rows > limit) P_rows = limit;
+  } else if (LN && MIN_CTAS == 2 && p.R <= 2 * sms && P_rows > sms) {
+    P_rows = sms;
+  }
   norm_bwd_kernel<LN, STATS, T, VPT, NT, MIN_CTAS><<<static_cast<unsigned>(P_rows), NT, 0, stream>>>(p);
 }
 
@@ -476,19 +488,34 @@ static void launch_norm_bwd_width(const NormBwdParams& p, int64_t nvec, int64_t&
   //   8192 x 4096 fp32          88.1 / 85.7                73.1 / 73.6
   //   8192 x 12288  (4, 512, 1) 213.7 / 129.8  (2, 1024, 1) 262.2 / 198.6  scalar path 875 / 831
   //   8192 x 5120 fp32          107.2 / 104.4               125.0 / 117.5              387 / 356
+  // With few rows the time of one row counts, and RMSNorm, whose sums leave registers for it, takes
+  // more threads per row. RMSNorm / act(RMSNorm), statistics recomputed, bf16 unless noted:
+  //   1000 x 2048  (2, 128, 5) 11.9 / 14.1  (1, 256, 3) 9.4 / 11.0    4500 x 2048 18.0 / 25.7  18.7 / 25.4
+  //   296 x 6144   (3, 256, 2) 10.7 / 12.3  (2, 512, 1) 9.8 / 11.7    500 x 6144 11.9 / 15.0  12.7 / 16.4
+  //   148 x 8192   (4, 256, 2) 9.4 / 12.3   (2, 512, 1) 9.0 / 10.2    1000 x 8192 18.9 / 29.1  19.8 / 27.3
+  //   148 x 4096 fp32          7.0 / 9.0                7.0 / 8.0     500 x 4096 10.5 / 14.5  11.3 / 15.5
   constexpr bool F32 = Pack<T>::VEC == 4;
-  constexpr int V256 = LN || !F32 ? 2 : 1;
-  if (nvec <= 64) launch_norm_bwd_vec<LN, STATS, T, 1, 64, 12>(p, P_rows, stream);
-  else if (nvec <= 128) launch_norm_bwd_vec<LN, STATS, T, 1, 128, 6>(p, P_rows, stream);
-  else if (nvec <= 256) launch_norm_bwd_vec<LN, STATS, T, V256, 256 / V256, V256 == 2 ? 5 : 3>(p, P_rows, stream);
-  else if (nvec <= 512) launch_norm_bwd_vec<LN, STATS, T, LN ? 4 : 2, LN ? 128 : 256, 3>(p, P_rows, stream);
-  else if (nvec <= 768) launch_norm_bwd_vec<LN, STATS, T, 3, 256, 2>(p, P_rows, stream);
-  else if (nvec <= 1024) {
-    if constexpr (LN && !F32) launch_norm_bwd_vec<LN, STATS, T, 2, 512, 1>(p, P_rows, stream);
-    else launch_norm_bwd_vec<LN, STATS, T, 4, 256, 2>(p, P_rows, stream);
-  } else {
-    launch_norm_bwd_vec<LN, STATS, T, 4, 512, 1>(p, P_rows, stream);
+  const int64_t sms = sm_count_of_current_device();
+  if (nvec <= 64) return launch_norm_bwd_vec<LN, STATS, T, 1, 64, 12>(p, P_rows, stream);
+  if (nvec <= 128) return launch_norm_bwd_vec<LN, STATS, T, 1, 128, 6>(p, P_rows, stream);
+  if (nvec <= 256) {
+    if constexpr (!LN)
+      if (F32 || p.R < 16 * sms) return launch_norm_bwd_vec<LN, STATS, T, 1, 256, 3>(p, P_rows, stream);
+    if constexpr (LN || !F32) return launch_norm_bwd_vec<LN, STATS, T, 2, 128, 5>(p, P_rows, stream);
   }
+  if (nvec <= 512)
+    return launch_norm_bwd_vec<LN, STATS, T, LN ? 4 : 2, LN ? 128 : 256, 3>(p, P_rows, stream);
+  if constexpr (!LN) {
+    const int64_t few = nvec <= 768 || F32 ? 2 : p.act >= 0 ? 8 : 4;
+    if (nvec <= 1024 && p.R <= few * sms)
+      return launch_norm_bwd_vec<LN, STATS, T, 2, 512, 1>(p, P_rows, stream);
+  }
+  if (nvec <= 768) return launch_norm_bwd_vec<LN, STATS, T, 3, 256, 2>(p, P_rows, stream);
+  if (nvec <= 1024) {
+    if constexpr (LN && !F32) return launch_norm_bwd_vec<LN, STATS, T, 2, 512, 1>(p, P_rows, stream);
+    else return launch_norm_bwd_vec<LN, STATS, T, 4, 256, 2>(p, P_rows, stream);
+  }
+  launch_norm_bwd_vec<LN, STATS, T, 4, 512, 1>(p, P_rows, stream);
 }
 
 template <bool LN, typename T>
