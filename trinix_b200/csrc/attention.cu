@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const float slope2 = p.slopes ? p.slopes[hq] * 1.4426950408889634f : 0.0f;
     const bool has_alibi = p.slopes != nullptr;
     constexpr bool has_bias = feature_has_mask(FEATURE);
-    const bool has_drop = FEATURE != ATT_PLAIN && p.drop_thr != 0u;
+    const bool has_drop = FEATURE == ATT_DROPOUT || (has_bias && p.drop_thr != 0u);
     // The mask values of this warp's 16 rows come into shared memory by cp.async, 32 columns (one
     // chunk of 16 rows x 128 bytes) at a time and MASK_BUFS chunks ahead of their use: a copy of the
     // warp covers whole row segments (one or two cache lines each, any alignment), and its latency
@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       const uint8_t* src = reinterpret_cast<const uint8_t*>(p.bias) +
                            ESZ * (b * p.bias_sb + hq * p.bias_sh + (mask_row0 + r0) * p.bias_sq +
                                   (live > 0 ? col : 0));
-      const uint32_t dst = mask_ring + (n % L::MASK_BUFS) * L::MASK_CHUNK + r0 * 128 +
+      const uint32_t dst = mask_ring + (n & (L::MASK_BUFS - 1)) * L::MASK_CHUNK + r0 * 128 +
                            (((c >> 3) ^ (r0 & 3)) << 5) + (c & 7) * ESZ;
       const int rows = p.Sq - mask_row0 - r0;  // of the mask from this lane's first one on
 #pragma unroll
@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         else if (c0 >= row1) alibi_sgn = -1;          // every key at or after every query
       }
       // general path: a tile that straddles the diagonal under ALiBi, or a non-positive scale
-      const bool general = (has_alibi && alibi_sgn == 0) || !(sl2 > 0.0f) || has_drop;
+      const bool general = (has_alibi && alibi_sgn == 0) || !(sl2 > 0.0f);
       float m_tile[2] = {-INFINITY, -INFINITY};
       float off[2] = {0.0f, 0.0f};  // fast path: x = t * sl2 + off
       auto max_of_tile = [&](float unit) {  // of scores that become x = t * unit + off
@@ -830,49 +830,65 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
           m_tile[hr] = (mraw == -INFINITY) ? -INFINITY : fmaf(mraw, unit, off[hr]);
         }
       };
-      if constexpr (has_bias) {
-        // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf
+      if constexpr (FEATURE != ATT_PLAIN) {
+        // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf. Dropout without a
+        // mask does the same, every path fixed at compile time: 2 x 4096^2, 16 / 4 heads, head dim
+        // 128, 858 us (causal 523). Left to run-time flags beside the plain paths its 96 registers
+        // spill in the generator's loop: 1470 us (887); one instantiation for masks and dropout with
+        // a flag for each: 1097 us (673).
         const float2 scale2 = make_float2(sl2, sl2);
-        const float2 log2e2 = make_float2(1.4426950408889634f, 1.4426950408889634f);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(L::MASK_BUFS - 1) : "memory");
-          __syncwarp();
-          const int n = 4 * itn + c;
-          const uint32_t from = mask_ring + (c % L::MASK_BUFS) * L::MASK_CHUNK + (lane >> 2) * 128;
-#pragma unroll
-          for (int g = 4 * c; g < 4 * c + 4; ++g) {
-            const uint32_t at = from + (((g & 3) ^ ((lane >> 2) & 3)) << 5);
-#pragma unroll
-            for (int hr = 0; hr < 2; ++hr) {
-              float2 bv;
-              if constexpr (FEATURE == ATT_MASK_F32) {
-                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                             : "=f"(bv.x), "=f"(bv.y)
-                             : "r"(at + hr * 1024 + q4 * 8)
-                             : "memory");
-              } else {
-                uint32_t u;
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"(at + hr * 1024 + q4 * 4)
-                             : "memory");
-                bv = Pack<std::conditional_t<BF16, __nv_bfloat16, __half>>::cvt2(u);
-              }
-              const int i = 4 * g + 2 * hr;
-              float2 x = mul2(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), scale2);
-              if (has_alibi) {
-                const float d = static_cast<float>(row_g[hr] - c0 - 8 * g - 2 * q4);
-                x.x = fmaf(-slope2, fabsf(d), x.x);
-                x.y = fmaf(-slope2, fabsf(d - 1.0f), x.y);
-              }
-              x = fma2(bv, log2e2, x);
-              sr[i] = __float_as_uint(x.x);
-              sr[i + 1] = __float_as_uint(x.y);
-            }
+        auto scaled = [&](int g, int hr) {  // columns 8 g + 2 q4 + {0, 1}, without the mask
+          const int i = 4 * g + 2 * hr;
+          float2 x = mul2(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), scale2);
+          if (has_alibi) {
+            const float d = static_cast<float>(row_g[hr] - c0 - 8 * g - 2 * q4);
+            x.x = fmaf(-slope2, fabsf(d), x.x);
+            x.y = fmaf(-slope2, fabsf(d - 1.0f), x.y);
           }
-          __syncwarp();  // every lane has read the chunk
-          const int next = n + L::MASK_BUFS;
-          if (next < 4 * n_it) copy_mask(next, j_first + (next >> 2) * kv_step);
-          mask_commit();
+          return x;
+        };
+        auto store = [&](int g, int hr, float2 x) {
+          sr[4 * g + 2 * hr] = __float_as_uint(x.x);
+          sr[4 * g + 2 * hr + 1] = __float_as_uint(x.y);
+        };
+        if constexpr (has_bias) {
+          const float2 log2e2 = make_float2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(L::MASK_BUFS - 1) : "memory");
+            __syncwarp();
+            const int n = 4 * itn + c;
+            const uint32_t from = mask_ring + (c % L::MASK_BUFS) * L::MASK_CHUNK + (lane >> 2) * 128;
+#pragma unroll
+            for (int g = 4 * c; g < 4 * c + 4; ++g) {
+              const uint32_t at = from + (((g & 3) ^ ((lane >> 2) & 3)) << 5);
+#pragma unroll
+              for (int hr = 0; hr < 2; ++hr) {
+                float2 bv;
+                if constexpr (FEATURE == ATT_MASK_F32) {
+                  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                               : "=f"(bv.x), "=f"(bv.y)
+                               : "r"(at + hr * 1024 + q4 * 8)
+                               : "memory");
+                } else {
+                  uint32_t u;
+                  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"(at + hr * 1024 + q4 * 4)
+                               : "memory");
+                  bv = Pack<std::conditional_t<BF16, __nv_bfloat16, __half>>::cvt2(u);
+                }
+                store(g, hr, fma2(bv, log2e2, scaled(g, hr)));
+              }
+            }
+            __syncwarp();  // every lane has read the chunk
+            const int next = n + L::MASK_BUFS;
+            if (next < 4 * n_it) copy_mask(next, j_first + (next >> 2) * kv_step);
+            mask_commit();
+          }
+        } else {
+#pragma unroll
+          for (int g = 0; g < 16; ++g)
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) store(g, hr, scaled(g, hr));
         }
         if (need_mask) {
 #pragma unroll
@@ -989,7 +1005,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       // P = exp2(x - m_ref), packed to 16-bit pairs IN PLACE: sr[2g + hr] = P(row hr, column
       // 4g + q4). Slot 2g + hr never lies ahead of the scores still to be read (4g + 2hr ..).
       float2 lsum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-      if (has_bias ? has_drop : general) {
+      if (FEATURE == ATT_PLAIN ? general : has_drop) {
         uint4 rnd[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
 #pragma unroll
         for (int g = 0; g < 16; ++g) {
@@ -1093,7 +1109,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       const float l_row = xch[r];
       const float m_row = xch[ATT_BM + r];
       float inv = (n_it > 0 && l_row > 0.0f) ? __fdividef(1.0f, l_row) : 0.0f;
-      if (FEATURE != ATT_PLAIN && p.drop_thr != 0u) inv *= p.drop_scale;  // kept probabilities count 1 / (1 - p)
+      if (has_drop) inv *= p.drop_scale;  // kept probabilities count 1 / (1 - p)
       const uint32_t o_addr = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + 2 * ATT_BN +
                               t * ATT_BN + sub * OC;
       uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) +
