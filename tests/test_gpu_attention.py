@@ -359,16 +359,17 @@ def test_dense_mask_rejects_bad_shapes(cuda):
 
 def test_launch_after_recorded_failure_raises_then_recovers(cuda):
     """A non-zero status word (a bounded wait gave up in some earlier launch) makes every later
-    launch skip its work on the device. The host learns of it without a synchronisation: every
-    attention call queues a 4-byte copy of the word into pinned memory and the next call checks
-    that copy first, raising status -8 instead of handing back unwritten output. The word is set
-    from the host here; no wait on the device is ever made to run out."""
+    launch skip its work on the device. The host learns of it without a synchronisation: a launch
+    that skips its work (or gives up) writes the word into the pinned host memory attached to the
+    workspace and the next call checks that first, raising status -8 instead of handing back
+    unwritten output. The word is set from the host here; no wait on the device is ever made to
+    run out."""
     from trinix_b200 import ops
     q, k, v = (t.to(cuda) for t in _qkv(1, 512, 512, 4, 2, 128, seed=21))
     good = T.attention(q, k, v, causal=True)
     assert T.attention_status(cuda) == 0
     ops._workspace(cuda)[:4].view(torch.int32).fill_(4)     # as if a softmax wait had run out
-    T.attention(q, k, v, causal=True)                        # skipped on the device; copy queued
+    T.attention(q, k, v, causal=True)                        # skipped on the device; word written
     torch.cuda.synchronize(cuda)
     with pytest.raises(T._lib.TrinixB200Error) as e:         # first call that can know: raises
         T.attention(q, k, v, causal=True)
