@@ -400,8 +400,9 @@ int trx_attn_status(const void* workspace, unsigned int* host_word, void* stream
  * bounded wait, or that finds such a failure recorded and skips its work, also writes the status
  * word there; a launch that works touches nothing. A host that reads the word before each call
  * needs no trx_attn_status copies. The caller keeps the word alive as long as it is attached, and
- * zeroes it together with the device word. One small launch on `stream`. Replaces nothing in the
- * reference.
+ * after a failure zeroes the device word first and this one when no launch queued before that is
+ * left (each of them reports the failure again). One small launch on `stream`. Replaces nothing in
+ * the reference.
  */
 int trx_attn_mirror(void* workspace, unsigned int* host_word_or_null, void* stream);
 
