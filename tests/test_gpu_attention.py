@@ -536,6 +536,55 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hk,D,causal,window,alibi,scale", [
+    (40, 130, 130, 8, 8, 128, False, None, False, None),   # two rows in the second Q tile
+    (40, 100, 300, 8, 8, 64, True, None, False, None),     # none
+    (13, 700, 700, 24, 8, 128, True, None, False, None),   # row pairs, one to six KV tiles each
+    (6, 1500, 1500, 16, 4, 128, True, None, False, None),  # pairs of heads
+    (20, 1000, 1000, 8, 8, 64, False, (200, 0), False, None),   # tiles that start one later
+    (20, 600, 600, 8, 8, 128, False, (30, 150), False, None),   # hidden at both ends
+    (30, 700, 130, 8, 8, 64, False, (10, 3), False, None),      # items and rows without any key
+    (30, 300, 0, 8, 8, 128, False, None, False, None),          # no key at all
+    (20, 513, 513, 8, 2, 128, False, None, True, None),    # ALiBi on both sides of the query
+    (20, 513, 513, 8, 8, 64, True, None, True, None),      # before it: last tile first, row pairs
+    (20, 400, 400, 8, 2, 128, False, None, False, -0.1),   # a scale that is not positive
+    (20, 700, 700, 8, 2, 128, False, None, False, 1.5),    # large scores: O is rescaled
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_more_work_items_than_ctas(cuda, B, Sq, Sk, Hq, Hk, D, causal, window, alibi, scale, dtype):
+    """Every CTA works on several items, of different lengths and with Q tiles that differ in their
+    keys. Reference in fp32 on the device; the log sums' bound is relative to the scores."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(B, Sq, Sk, Hq, Hk, D, seed=Sq + Sk, dtype=dtype))
+    slopes = R.alibi_slopes_ref(Hq).to(cuda) if alibi else None
+    out, lse = ops.attention(q, k, v, causal=causal, scale=scale, window=window,
+                             alibi_slopes=slopes, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    g = Hq // Hk
+    s = torch.einsum("bihd,bjhd->bhij", q.float(), k.float().repeat_interleave(g, 2))
+    s = s * (D ** -0.5 if scale is None else scale)
+    i, j = torch.arange(Sq, device=cuda)[:, None], torch.arange(Sk, device=cuda)[None]
+    if slopes is not None:
+        s = s - slopes.view(1, -1, 1, 1) * (i - j).abs()
+    if causal:
+        s = s.masked_fill(j > i, float("-inf"))
+    if window is not None:
+        s = s.masked_fill((j - i < -window[0]) | (j - i > window[1]), float("-inf"))
+    ref_lse = torch.logsumexp(s, -1)
+    seen = ~torch.isinf(ref_lse)
+    assert torch.equal(torch.isinf(lse), ~seen)
+    if seen.any():
+        largest = max(1.0, float(s[~torch.isinf(s)].abs().max()))
+        assert float((lse[seen] - ref_lse[seen]).abs().max()) <= 1e-5 * (5 + largest)
+        p, vt = torch.softmax(s, -1).nan_to_num_(0.0), v.float().repeat_interleave(g, 2)
+        ref = torch.einsum("bhij,bjhd->bihd", p, vt)
+        # probabilities and the result are each rounded to u of themselves
+        u = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+        bound = u * (ref.abs() + torch.einsum("bhij,bjhd->bihd", p, vt.abs())) + 1e-4
+        assert bool(((out.float() - ref).abs() <= bound).all())
+    assert not out[~seen.transpose(1, 2)].any()
+
+
 @pytest.mark.parametrize("Sq", [1, 4])
 def test_few_query_rows_in_every_layout(cuda, Sq):
     """The same call with contiguous tensors, transposed (B, H, S, D) storage, a slice of a longer

@@ -1,4 +1,6 @@
-// Attention forward for sm_100a: softmax(scale * Q K^T + bias) V with online softmax.
+// Attention forward with a dense additive mask or dropout, and the host side of every attention call:
+// softmax(scale * Q K^T + bias) V with online softmax. Calls without either run attention_plain.cu or,
+// with up to 16 query rows, attention_decode.cuh (but for a few, see use_decode).
 //
 // One CTA owns two 128-row Q tiles that ping-pong on the tensor pipe: the same 128 query rows of
 // two query heads that share a kv head (GQA / MQA: both tiles then see exactly the same keys), or
@@ -21,334 +23,16 @@
 // h / (Hq / Hk), so GQA / MQA need no tiled copies. With ALiBi under a causal mask the KV tiles
 // of a row block are visited from the diagonal backwards: the bias grows with the key index, so
 // in that order the first tile holds the row maximum and O is never rescaled again.
-// Calls of up to 16 query rows without mask or dropout take the kernel of attention_decode.cuh (but
-// for a few, see use_decode).
 //
 // Every wait on an mbarrier is bounded: after a fixed number of polls the kernel records a
 // code in the status word of the caller's workspace, raises a CTA-wide abort flag, drains its
 // own copies and MMAs (bounded again), frees its TMEM and returns.
-#include <cuda.h>
-
-#include <atomic>
-#include <mutex>
-#include <type_traits>
-
-#include "common.cuh"
+#include "attention_common.cuh"
 
 namespace trx {
 
-constexpr int ATT_BM = 128;       // rows per Q tile
-constexpr int ATT_BN = 128;       // keys per KV tile
-constexpr int ATT_NQ = 2;         // Q tiles per CTA
-constexpr int ATT_STAGES = 4;     // KV ring depth (K and V tiles alternate)
-constexpr int ATT_SM_WARPS = 16;    // softmax warps: two warpgroups per Q tile, half a row per thread
-constexpr int ATT_THREADS = (ATT_SM_WARPS + 2) * 32;
-constexpr uint32_t ATT_WAIT_LIMIT = 1u << 26;  // hard cap on polls per wait
-constexpr uint64_t ATT_WAIT_NS = 400ull * 1000 * 1000;  // wall-time budget of one wait
-constexpr float ATT_LAZY_RESCALE = 8.0f;       // log2 units
-
-enum AttnStatus : unsigned {
-  ATT_ST_PRODUCER = 1u,
-  ATT_ST_MMA = 2u,
-  ATT_ST_SOFTMAX = 4u,
-  ATT_ST_DRAIN = 8u,
-};
-
-struct AttnParams {
-  CUtensorMap tm_q;
-  CUtensorMap tm_k;
-  CUtensorMap tm_v;
-  void* out;
-  float* lse;
-  const float* slopes;
-  unsigned int* status;
-  int B, Sq, Sk, Hq;
-  int k_hdiv, v_hdiv;  // query heads per kv head (Hq when the tensor's heads are collapsed)
-  int k_bmul, v_bmul;  // 1, or 0 when the batch dim is broadcast
-  int group;           // consecutive query heads that read one kv head in K and in V
-  int decode;          // few query rows: attention_decode.cuh
-  const void* q;       // read directly by the decode kernel
-  long long q_stride_b, q_stride_s, q_stride_h;
-  long long o_stride_b, o_stride_s, o_stride_h;
-  long long lse_stride_b, lse_stride_h;
-  float scale_log2;    // softmax scale * log2(e)
-  int causal;
-  int win_left, win_right;  // < 0: no window
-  int is_bf16;
-  int reverse_m;       // schedule the heaviest (last) row blocks first
-  int reverse_kv;      // visit a row block's KV tiles from the last to the first
-  int pair_heads;      // the two Q tiles of a CTA: same 128 rows of two query heads that share a
-                       // kv head (1), or two consecutive 128-row blocks of one head (0)
-  // dense additive mask (B, Hq, Sq, Sk) with unit key stride; batch / head strides may be 0
-  const void* bias;
-  long long bias_sb, bias_sh, bias_sq;  // elements
-  int bias_kind;       // 0 none, 1 fp32, 2 the activation dtype
-  int bias_copy;       // bytes of one copy that every row's alignment allows: 16, 4 or 2
-  // dropout on the normalised probabilities: an element is dropped when its random byte is
-  // below drop_thr (0 = no dropout); kept ones are scaled by drop_scale = 256 / (256 - drop_thr)
-  unsigned drop_thr;
-  float drop_scale;
-  unsigned seed_lo, seed_hi, drop_offset;
-};
-
-// Philox4x32-10 (Salmon et al., "Parallel random numbers: as easy as 1, 2, 3", 2011): a counter
-// based generator, so that any element's random byte can be recomputed anywhere, on the host
-// too. The dropout stream is keyed by the caller's 64-bit seed; the counter is
-// (key index / 16, query row, batch * heads + head, offset) and the 16 bytes of the result
-// belong to the 16 consecutive keys of that block, least significant byte first.
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1) {
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-    c = make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
-  }
-  return c;
-}
-
-// ------------------------------------------------------------------------------------------
-// PTX wrappers
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-// Bounded wait: gives up after ATT_WAIT_NS of wall time. Returns false if the CTA is aborting
-// (this wait ran out or another one did); the first to give up records `code` in the status word.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned int* status, unsigned code) {
-#pragma unroll 1
-  for (int fast = 0; fast < 64; ++fast)
-    if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
-#pragma unroll 1
-  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 63u) == 63u) {
-      if (*abort_flag) return false;
-      if (global_ns() - t0 > ATT_WAIT_NS) break;
-    }
-  }
-  *abort_flag = 1;
-  atomicOr(status, code);
-  return false;
-}
-// The status word's copy in host memory, if trx_attn_mirror attached one (workspace words 1 to 3:
-// a tag and the address). Written only by a launch that gave up or found a recorded failure, so a
-// launch that works pays nothing for it; a copy behind every launch, 4 bytes or not, holds the
-// stream for two hand-overs between the compute and the copy engine.
-constexpr unsigned ATT_MIRROR_TAG = 0x5452584du;
-__device__ __forceinline__ void report_status(unsigned int* status) {
-  if (status[1] != ATT_MIRROR_TAG) return;
-  volatile unsigned int* host = *reinterpret_cast<unsigned int* const*>(status + 2);
-  *host = *reinterpret_cast<volatile unsigned int*>(status);
-  __threadfence_system();
-}
-__global__ void attach_mirror_kernel(unsigned int* status, unsigned int* host) {
-  *reinterpret_cast<unsigned int**>(status + 2) = host;
-  status[1] = host ? ATT_MIRROR_TAG : 0u;
-}
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
-                                            int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      :
-      : "r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar)
-               : "memory");
-}
-// D[tmem] = A[smem] * B[smem]  (first) / D[tmem] += A[smem] * B[smem]  (acc)
-__device__ __forceinline__ void mma_ss_first(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                             uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-      : "memory");
-}
-__device__ __forceinline__ void mma_ss_acc(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                           uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]; `acc` = 0 overwrites D
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack16(float lo, float hi) {
-  if constexpr (BF16) return Pack<__nv_bfloat16>::pack2(lo, hi);
-  else return Pack<__half>::pack2(lo, hi);
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-// 2^x on the special-function unit; 2^-inf = +0.
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base lane + t).
-template <int OFF, int N>
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[N]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[OFF + 0]), "=r"(r[OFF + 1]), "=r"(r[OFF + 2]), "=r"(r[OFF + 3]), "=r"(r[OFF + 4]),
-        "=r"(r[OFF + 5]), "=r"(r[OFF + 6]), "=r"(r[OFF + 7]), "=r"(r[OFF + 8]), "=r"(r[OFF + 9]),
-        "=r"(r[OFF + 10]), "=r"(r[OFF + 11]), "=r"(r[OFF + 12]), "=r"(r[OFF + 13]),
-        "=r"(r[OFF + 14]), "=r"(r[OFF + 15]), "=r"(r[OFF + 16]), "=r"(r[OFF + 17]),
-        "=r"(r[OFF + 18]), "=r"(r[OFF + 19]), "=r"(r[OFF + 20]), "=r"(r[OFF + 21]),
-        "=r"(r[OFF + 22]), "=r"(r[OFF + 23]), "=r"(r[OFF + 24]), "=r"(r[OFF + 25]),
-        "=r"(r[OFF + 26]), "=r"(r[OFF + 27]), "=r"(r[OFF + 28]), "=r"(r[OFF + 29]),
-        "=r"(r[OFF + 30]), "=r"(r[OFF + 31])
-      : "r"(taddr)
-      : "memory");
-}
-template <int OFF, int N>
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[N]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      :
-      : "r"(taddr), "r"(r[OFF + 0]), "r"(r[OFF + 1]), "r"(r[OFF + 2]), "r"(r[OFF + 3]),
-        "r"(r[OFF + 4]), "r"(r[OFF + 5]), "r"(r[OFF + 6]), "r"(r[OFF + 7]), "r"(r[OFF + 8]),
-        "r"(r[OFF + 9]), "r"(r[OFF + 10]), "r"(r[OFF + 11]), "r"(r[OFF + 12]), "r"(r[OFF + 13]),
-        "r"(r[OFF + 14]), "r"(r[OFF + 15]), "r"(r[OFF + 16]), "r"(r[OFF + 17]), "r"(r[OFF + 18]),
-        "r"(r[OFF + 19]), "r"(r[OFF + 20]), "r"(r[OFF + 21]), "r"(r[OFF + 22]), "r"(r[OFF + 23]),
-        "r"(r[OFF + 24]), "r"(r[OFF + 25]), "r"(r[OFF + 26]), "r"(r[OFF + 27]), "r"(r[OFF + 28]),
-        "r"(r[OFF + 29]), "r"(r[OFF + 30]), "r"(r[OFF + 31])
-      : "memory");
-}
-// 16 lanes x 256 bits per repetition (8 fp32 columns). Thread t of the warp holds, for column
-// group g (8 columns each): r[4g+0..1] = lane (t/4), columns 8g + 2(t%4) + {0,1};
-// r[4g+2..3] = lane (t/4) + 8, same columns. Four threads (a quad) share a lane.
-__device__ __forceinline__ void tmem_ld_16x256b_x16(uint32_t taddr, uint32_t (&r)[64]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st_16x256b_x16(uint32_t taddr, const uint32_t (&r)[64]) {
-  asm volatile("tcgen05.st.sync.aligned.16x256b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63, %64};"
-               :
-               : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(r[32]), "r"(r[33]), "r"(r[34]), "r"(r[35]), "r"(r[36]), "r"(r[37]), "r"(r[38]), "r"(r[39]), "r"(r[40]), "r"(r[41]), "r"(r[42]), "r"(r[43]), "r"(r[44]), "r"(r[45]), "r"(r[46]), "r"(r[47]), "r"(r[48]), "r"(r[49]), "r"(r[50]), "r"(r[51]), "r"(r[52]), "r"(r[53]), "r"(r[54]), "r"(r[55]), "r"(r[56]), "r"(r[57]), "r"(r[58]), "r"(r[59]), "r"(r[60]), "r"(r[61]), "r"(r[62]), "r"(r[63])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st_16x256b_x8(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile("tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-               :
-               : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-               : "memory");
-}
-// 16 lanes x 128 bits per repetition (4 columns): r[2g+0] = lane (t/4), column 4g + (t%4);
-// r[2g+1] = lane (t/4) + 8, same column.
-template <int N>
-__device__ __forceinline__ void tmem_st_16x128b_x16(uint32_t taddr, const uint32_t (&r)[N]) {
-  asm volatile("tcgen05.st.sync.aligned.16x128b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-               :
-               : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field = 1.
-//   K-major operand : rows of 64 16-bit elements (128 B); 8-row groups 1024 B apart (SBO).
-//   MN-major operand: 64 contiguous MN elements per 128-B row of K; 8 K-rows per 1024-B group
-//                     (SBO); the next 64 MN elements start LBO bytes further.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes,
-                                              uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= 1ull << 46;  // descriptor version
-  d |= 2ull << 61;  // SWIZZLE_128B
-  return d;
-}
-// Instruction descriptor for kind::f16 with fp32 accumulation.
-__host__ __device__ constexpr uint32_t make_idesc(int is_bf16, int m, int n, int a_mn_major,
-                                                  int b_mn_major) {
-  return (1u << 4) |                                   // D format fp32
-         (static_cast<uint32_t>(is_bf16 ? 1 : 0) << 7) |   // A format
-         (static_cast<uint32_t>(is_bf16 ? 1 : 0) << 10) |  // B format
-         (static_cast<uint32_t>(a_mn_major) << 15) | (static_cast<uint32_t>(b_mn_major) << 16) |
-         (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-// What an instantiation carries: nothing beyond causal / window / ALiBi; dropout; a dense additive
-// mask with or without dropout.
-enum AttnFeature { ATT_PLAIN = 0, ATT_DROPOUT = 1, ATT_MASK_F32 = 2, ATT_MASK_16 = 3 };
+// What an instantiation carries: dropout; a dense additive mask with or without dropout.
+enum AttnFeature { ATT_DROPOUT = 1, ATT_MASK_F32 = 2, ATT_MASK_16 = 3 };
 __host__ __device__ constexpr bool feature_has_mask(int f) { return f >= ATT_MASK_F32; }
 
 // With a mask each softmax warp has MASK_BUFS buffers of 16 rows x 32 mask values; at head dim 128
@@ -371,25 +55,6 @@ struct AttnSmem {
   static constexpr int TOTAL = MASK_OFF + ATT_SM_WARPS * MASK_BUFS * MASK_CHUNK;
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for 1024-byte alignment
 };
-
-struct TileRange {
-  int jlo, jhi;  // KV tiles [jlo, jhi)
-};
-
-__device__ __forceinline__ TileRange tile_range(const AttnParams& p, int row0) {
-  TileRange r{0, 0};
-  if (row0 >= p.Sq) return r;
-  const int row1 = min(p.Sq, row0 + ATT_BM) - 1;
-  int hi = p.Sk - 1;
-  if (p.causal) hi = min(hi, row1);
-  if (p.win_right >= 0) hi = min(hi, row1 + p.win_right);
-  int lo = 0;
-  if (p.win_left >= 0) lo = max(0, row0 - p.win_left);
-  if (hi < lo) return r;
-  r.jlo = lo / ATT_BN;
-  r.jhi = hi / ATT_BN + 1;
-  return r;
-}
 
 template <int D, bool BF16, int FEATURE>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
@@ -802,21 +467,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       tmem_wait_ld();
 
       const bool need_mask = (c0 + ATT_BN - 1 > hi_min) || (c0 < lo_max);
-      // ALiBi on a tile that lies entirely on one side of the diagonal is linear in the
-      // column: -slope*|i-j| = sgn*slope*(j-i). It then folds into the raw score as
-      // t = s + (sgn*slope2/sl2)*c, and the per-tile, per-row constant `off` below.
-      int alibi_sgn = 0;
-      if (has_alibi) {
-        // under a causal mask (or a window that ends at the query) every VISIBLE key is at or
-        // before its query, on the diagonal tile too; hidden keys are masked anyway
-        if (p.causal || p.win_right == 0 || c0 + ATT_BN - 1 <= row0) alibi_sgn = 1;
-        else if (c0 >= row1) alibi_sgn = -1;          // every key at or after every query
-      }
-      // general path: a tile that straddles the diagonal under ALiBi, or a non-positive scale
-      const bool general = (has_alibi && alibi_sgn == 0) || !(sl2 > 0.0f);
       float m_tile[2] = {-INFINITY, -INFINITY};
-      float off[2] = {0.0f, 0.0f};  // fast path: x = t * sl2 + off
-      auto max_of_tile = [&](float unit) {  // of scores that become x = t * unit + off
+      auto max_of_tile = [&] {
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
           float mx0 = -INFINITY, mx1 = -INFINITY;
@@ -826,11 +478,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             mx1 = max3(mx1, __uint_as_float(sr[4 * g + 4 + 2 * hr]),
                        __uint_as_float(sr[4 * g + 5 + 2 * hr]));
           }
-          const float mraw = fmaxf(mx0, mx1);
-          m_tile[hr] = (mraw == -INFINITY) ? -INFINITY : fmaf(mraw, unit, off[hr]);
+          m_tile[hr] = fmaxf(mx0, mx1);
         }
       };
-      if constexpr (FEATURE != ATT_PLAIN) {
+      {
         // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf. Dropout without a
         // mask does the same, every path fixed at compile time: 2 x 4096^2, 16 / 4 heads, head dim
         // 128, 858 us (causal 523). Left to run-time flags beside the plain paths its 96 registers
@@ -901,83 +552,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
                 if (8 * g + e < lo_c || 8 * g + e > hi_c) sr[4 * g + 2 * hr + e] = 0xff800000u;
           }
         }
-        max_of_tile(1.0f);
-      } else if (general) {
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          const float fi = static_cast<float>(row_g[hr] - c0 - 2 * q4);
-#pragma unroll
-          for (int g = 0; g < 16; ++g) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int i = 4 * g + 2 * hr + e;
-              float x = __uint_as_float(sr[i]) * sl2;
-              if (has_alibi) x = fmaf(-slope2, fabsf(fi - static_cast<float>(8 * g + e)), x);
-              if (need_mask) {
-                const int col = c0 + 8 * g + 2 * q4 + e;
-                if (col < lo_i[hr] || col > hi_i[hr]) x = -INFINITY;
-              }
-              sr[i] = __float_as_uint(x);
-              m_tile[hr] = fmaxf(m_tile[hr], x);
-            }
-          }
-        }
-      } else {
-        if (need_mask) {
-          // boundary tile: hide keys outside [lo, hi] in the raw domain (sl2 > 0 keeps -inf
-          // at -inf), then continue on the fast path
-          // a tile is cut by the upper bound (diagonal), by the lower one (left edge of a
-          // window), seldom by both: one comparison per score where one is enough
-          const bool cut_hi = c0 + ATT_BN - 1 > hi_min, cut_lo = c0 < lo_max;
-#pragma unroll
-          for (int hr = 0; hr < 2; ++hr) {
-            const int lo_c = lo_i[hr] - c0 - 2 * q4, hi_c = hi_i[hr] - c0 - 2 * q4;
-            if (cut_hi && !cut_lo) {
-#pragma unroll
-              for (int g = 0; g < 16; ++g) {
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                  if (8 * g + e > hi_c) sr[4 * g + 2 * hr + e] = 0xff800000u;
-              }
-            } else if (cut_lo && !cut_hi) {
-#pragma unroll
-              for (int g = 0; g < 16; ++g) {
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                  if (8 * g + e < lo_c) sr[4 * g + 2 * hr + e] = 0xff800000u;
-              }
-            } else {
-#pragma unroll
-              for (int g = 0; g < 16; ++g) {
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                  if (8 * g + e < lo_c || 8 * g + e > hi_c) sr[4 * g + 2 * hr + e] = 0xff800000u;
-              }
-            }
-          }
-        }
-        if (alibi_sgn != 0) {
-          const float sk = static_cast<float>(alibi_sgn) * slope2;
-          const float kc = __fdividef(sk, sl2);
-#pragma unroll
-          for (int hr = 0; hr < 2; ++hr)
-            off[hr] = sk * static_cast<float>(c0 + 2 * q4 - row_g[hr]);
-          // + kc * (8g + e), as packed adds of a running (column, column + 1) pair
-          float2 cp = make_float2(0.0f, kc);
-          const float2 step = make_float2(8.0f * kc, 8.0f * kc);
-#pragma unroll
-          for (int g = 0; g < 16; ++g) {
-#pragma unroll
-            for (int hr = 0; hr < 2; ++hr) {
-              const float2 v = add2(make_float2(__uint_as_float(sr[4 * g + 2 * hr]),
-                                                __uint_as_float(sr[4 * g + 2 * hr + 1])), cp);
-              sr[4 * g + 2 * hr] = __float_as_uint(v.x);
-              sr[4 * g + 2 * hr + 1] = __float_as_uint(v.y);
-            }
-            cp = add2(cp, step);
-          }
-        }
-        max_of_tile(sl2);
+        max_of_tile();
       }
       // the four threads of a quad hold the four column slices of the same two rows
 #pragma unroll
@@ -1005,7 +580,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       // P = exp2(x - m_ref), packed to 16-bit pairs IN PLACE: sr[2g + hr] = P(row hr, column
       // 4g + q4). Slot 2g + hr never lies ahead of the scores still to be read (4g + 2hr ..).
       float2 lsum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-      if (FEATURE == ATT_PLAIN ? general : has_drop) {
+      if (has_drop) {
         uint4 rnd[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
 #pragma unroll
         for (int g = 0; g < 16; ++g) {
@@ -1035,17 +610,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
           }
         }
       } else {
-        const float unit = has_bias ? 1.0f : sl2;  // a mask's scores are scaled already
-        const float2 sc2 = make_float2(unit, unit);
-        const float2 nm2[2] = {make_float2(off[0] - m_ref[0], off[0] - m_ref[0]),
-                               make_float2(off[1] - m_ref[1], off[1] - m_ref[1])};
+        const float2 nm2[2] = {make_float2(-m_ref[0], -m_ref[0]),
+                               make_float2(-m_ref[1], -m_ref[1])};
 #pragma unroll
         for (int g = 0; g < 16; ++g) {
 #pragma unroll
           for (int hr = 0; hr < 2; ++hr) {
-            const float2 x = fma2(make_float2(__uint_as_float(sr[4 * g + 2 * hr]),
+            const float2 x = add2(make_float2(__uint_as_float(sr[4 * g + 2 * hr]),
                                               __uint_as_float(sr[4 * g + 2 * hr + 1])),
-                                  sc2, nm2[hr]);
+                                  nm2[hr]);
             const float2 pe = make_float2(fast_exp2(x.x), fast_exp2(x.y));
             lsum[hr] = add2(lsum[hr], pe);
             sr[2 * g + hr] = pack16<BF16>(pe.x, pe.y);
@@ -1260,8 +833,7 @@ template <int D, bool BF16>
 static int launch_attn(const AttnParams& p, cudaStream_t stream) {
   if (p.bias_kind == 1) return launch_attn_feature<D, BF16, ATT_MASK_F32>(p, stream);
   if (p.bias_kind == 2) return launch_attn_feature<D, BF16, ATT_MASK_16>(p, stream);
-  if (p.drop_thr != 0u) return launch_attn_feature<D, BF16, ATT_DROPOUT>(p, stream);
-  return launch_attn_feature<D, BF16, ATT_PLAIN>(p, stream);
+  return launch_attn_feature<D, BF16, ATT_DROPOUT>(p, stream);
 }
 
 }  // namespace trx
@@ -1269,6 +841,13 @@ static int launch_attn(const AttnParams& p, cudaStream_t stream) {
 #include "attention_decode.cuh"
 
 using namespace trx;
+
+namespace trx {
+__global__ void attach_mirror_kernel(unsigned int* status, unsigned int* host) {
+  *reinterpret_cast<unsigned int**>(status + 2) = host;
+  status[1] = host ? ATT_MIRROR_TAG : 0u;
+}
+}  // namespace trx
 
 extern "C" size_t trx_attn_workspace_bytes(void) { return 256; }
 
@@ -1336,7 +915,8 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   p.Hq = static_cast<int>(Hq);
   // two query heads per CTA when each pair (2i, 2i + 1) reads one kv head in K and in V
   p.pair_heads = (Hq % 2 == 0 && p.k_hdiv % 2 == 0 && p.v_hdiv % 2 == 0) ? 1 : 0;
-  p.decode = !bias && dropout_p == 0.0f && use_decode(p, D) ? 1 : 0;
+  p.plain = (!bias || Sk == 0) && dropout_p == 0.0f ? 1 : 0;
+  p.decode = p.plain && !bias && use_decode(p, D) ? 1 : 0;
   const int kv_box = p.decode ? DEC_KEYS : ATT_BN;
   rc = make_map(&p.tm_k, kk, is_bf16, D, Sk_map, k_hb ? 1 : Hk, k_bb ? 1 : B, k_strides[0],
                 k_strides[1], k_strides[2], kv_box);
@@ -1396,7 +976,7 @@ static int attn_fwd_prepare(AttnParams& p, bool* nothing_to_do, const void* q, c
   return TRX_OK;
 }
 
-static int attn_fwd_launch(const AttnParams& p, int64_t D, void* stream) {
+static int attn_fwd_launch(AttnParams& p, int64_t D, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (p.decode) {
     const bool wide = p.group * p.Sq > 16;
@@ -1406,6 +986,7 @@ static int attn_fwd_launch(const AttnParams& p, int64_t D, void* stream) {
     return p.is_bf16 ? (wide ? launch_decode<64, true, 2>(p, s) : launch_decode<64, true, 1>(p, s))
                      : (wide ? launch_decode<64, false, 2>(p, s) : launch_decode<64, false, 1>(p, s));
   }
+  if (p.plain) return launch_attn_plain(p, D, s);
   if (D == 128) return p.is_bf16 ? launch_attn<128, true>(p, s) : launch_attn<128, false>(p, s);
   return p.is_bf16 ? launch_attn<64, true>(p, s) : launch_attn<64, false>(p, s);
 }
