@@ -25,7 +25,7 @@
 //   * the issuing warps stay converged and elect a lane, and every branch goes by a vote: descriptors
 //     are then uniform registers (from one lane in divergent code 4 x 4096 full: 1142 us, so 991);
 //   * one issuing warp per Q tile: a wait on a ready barrier costs such a warp some 200 cycles, and
-//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1904;
+//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1874;
 //     window 1024: 1304, 1097; 8 x 2048 causal, 16 heads x 64: 188, 137);
 //   * cut tiles: one uniform test per visit, then bit masks (2900 -> 600 cycles for such a tile).
 // Measured and not taken: S shared by both tiles with P beside it (1016-1200 us on 4 x 4096 full
@@ -38,11 +38,6 @@ namespace trx {
 
 constexpr int AP_THREADS = 512;
 constexpr int AP_STAGES = 4;  // K / V ring
-// Registers per thread after the split. The four warpgroups' shares sum to what the launch gives
-// (4 x 128): 176 hold 128 scores; with 168 the loop spills (causal 16 x 4096: 2111 us against 1904),
-// 184 and 192 measured the same.
-constexpr int AP_R_SOFTMAX = 176, AP_R_EPILOGUE = 80, AP_R_OTHER = 80;
-static_assert(2 * AP_R_SOFTMAX + AP_R_EPILOGUE + AP_R_OTHER <= 512, "register split");
 // P is handed over in two pieces: the P V of the first 96 keys runs while the last 32 are
 // exponentiated (causal 16 x 4096: 1994 us in one piece, 1904 so, 2064 in halves).
 constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
@@ -50,6 +45,18 @@ constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
 // What is added to the scaled scores: nothing; ALiBi as one ramp per row (every visible key at or
 // before its query); ALiBi on either side of the query, or a scale that is not positive.
 enum AttnBias { AP_NONE = 0, AP_RAMP = 1, AP_GENERAL = 2 };
+
+// Registers per thread after the split. The four warpgroups' shares sum to what the launch gives
+// (4 x 128). The softmax loop holds 128 scores: with 168 it spills (16 x 4096 causal 2111 us against
+// 1947 with 176). Beyond that the register allocator's schedule decides, measured with 176 / 184:
+// plain scores at head dim 128: causal 1947 / 1874 us, window 1024 1189 / 1044, 2 x 8192 full 1953 /
+// 1731; with ALiBi 2153 / 2345; head dim 64, 8 x 2048 x 16 heads 226 / 239, causal 146 / 151.
+template <int D, int BIAS>
+struct PlainRegs {
+  static constexpr int SOFTMAX = D == 128 && BIAS == AP_NONE ? 184 : 176;
+  static constexpr int EPILOGUE = 256 - SOFTMAX, OTHER = 256 - SOFTMAX;
+  static_assert(2 * SOFTMAX + EPILOGUE + OTHER <= 512, "register split");
+};
 
 // Column numbers of a KV tile in pairs, for ALiBi's ramp: as immediates they cost two moves a pair
 // (16 x 4096 causal with ALiBi: 2490 us against 2262).
@@ -340,7 +347,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
   };
 
   if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AP_R_OTHER));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::OTHER));
     if (warp == 12) {
       // =========================== TMA producer =======================================
       if (lane == 0) {
@@ -602,7 +609,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     }
   } else if (warp >= 8) {
     // =========================== epilogue =============================================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AP_R_EPILOGUE));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::EPILOGUE));
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
     uint32_t opar[2] = {0u, 0u};  // parity of the next finished O
@@ -688,7 +695,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     }
   } else {
     // =========================== softmax ==============================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AP_R_SOFTMAX));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::SOFTMAX));
     const int t = warp >> 2;
     const int wq = warp & 3;
     const int rl = wq * 32 + lane;
@@ -898,7 +905,8 @@ static int launch_plain(const AttnParams& p, cudaStream_t stream) {
     if (cudaFuncGetAttributes(&a, attn_plain_kernel<D, BF16, BIAS>) != cudaSuccess)
       return TRX_ERR_CUDA;
     // the register split draws on what the block is launched with: never wait for more than that
-    if (a.numRegs * 4 < 2 * AP_R_SOFTMAX + AP_R_EPILOGUE + AP_R_OTHER) return TRX_ERR_UNSUPPORTED;
+    using Regs = PlainRegs<D, BIAS>;
+    if (a.numRegs * 4 < 2 * Regs::SOFTMAX + Regs::EPILOGUE + Regs::OTHER) return TRX_ERR_UNSUPPORTED;
     if (cudaFuncSetAttribute(attn_plain_kernel<D, BF16, BIAS>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              PlainSmem<D>::DYN_BYTES) != cudaSuccess)
