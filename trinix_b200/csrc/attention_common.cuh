@@ -54,8 +54,9 @@ struct AttnParams {
   int reverse_kv;      // visit a row block's KV tiles from the last to the first
   int pair_heads;      // the two Q tiles of a CTA: same 128 rows of two query heads that share a
                        // kv head (1), or two consecutive 128-row blocks of one head (0)
-  // order of the work items of attention_plain.cu (a 1-D grid)
-  int m_blocks, slots, slot_group;
+  // attention_plain.cu: which grid dimension counts row blocks, heads (or pairs) and batches; no more
+  // CTAs than SMs, so that each has one work item
+  int order, single;
   // dense additive mask (B, Hq, Sq, Sk) with unit key stride; batch / head strides may be 0
   const void* bias;
   long long bias_sb, bias_sh, bias_sq;  // elements
@@ -106,6 +107,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Without the suspension of try_wait: whether the phase is complete now.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.b32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(bar), "r"(parity)

@@ -99,18 +99,20 @@ struct PlainItem {
   int lo[ATT_NQ], hi[ATT_NQ];
 };
 static_assert(sizeof(PlainItem) <= 64, "shared memory slot");
-__device__ __forceinline__ PlainItem plain_item(const AttnParams& p, int idx) {
+// Which of a block index's x, y, z are the row block, the head (or pair of heads) and the batch; x runs
+// fastest. Row blocks first: the K and V of few heads are at work at a time. Under a causal mask row
+// blocks differ in length: with the heads of a batch, or all heads of all batches, running faster than
+// the row blocks the heaviest come first and the CTAs end together.
+enum PlainOrder { AP_MHB = 0, AP_HMB = 1, AP_HBM = 2 };
+__device__ __forceinline__ PlainItem plain_item(const AttnParams& p, int x, int y, int z) {
   PlainItem w;
   w.valid = 1;
-  // order: groups of slots (a slot: one batch and head or pair of heads); in a group by row block
-  const int per_group = p.slot_group * p.m_blocks;
-  const int grp = idx / per_group, rem = idx - grp * per_group;
-  const int slot0 = grp * p.slot_group, slots = min(p.slot_group, p.slots - slot0);
-  const int mi = rem / slots, slot = slot0 + rem - mi * slots;
-  const int mblk = p.reverse_m ? p.m_blocks - 1 - mi : mi;
-  const int heads = p.pair_heads ? p.Hq / 2 : p.Hq;
-  w.b = slot / heads;
-  w.h = (slot - w.b * heads) * (p.pair_heads ? 2 : 1);
+  const int mi = p.order == AP_MHB ? x : p.order == AP_HMB ? y : z;
+  const int hi = p.order == AP_MHB ? y : x;
+  w.b = p.order == AP_HBM ? y : z;
+  const int m_blocks = p.order == AP_MHB ? gridDim.x : p.order == AP_HMB ? gridDim.y : gridDim.z;
+  const int mblk = p.reverse_m ? m_blocks - 1 - mi : mi;
+  w.h = hi * (p.pair_heads ? 2 : 1);
   w.m0 = mblk * (p.pair_heads ? ATT_BM : ATT_NQ * ATT_BM);
   TileRange r[ATT_NQ];
   int jlo = 1 << 30, jhi = 0;
@@ -142,19 +144,21 @@ __device__ __forceinline__ void request_block(uint32_t dst, uint32_t bar) {
       : "memory");
 }
 // Whether the answer is a block index, and which.
-__device__ __forceinline__ bool requested_block(uint32_t src, int& x) {
-  uint32_t ok, a;
+__device__ __forceinline__ bool requested_block(uint32_t src, int& x, int& y, int& z) {
+  uint32_t ok, a, b, c;
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
-      "ld.shared.b128 h, [%2];\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t.reg .b32 w;\n\t"
+      "ld.shared.b128 h, [%4];\n\t"
       "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
       "selp.b32 %0, 1, 0, p;\n\t"
-      "mov.b32 %1, 0;\n\t"
-      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
-      : "=r"(ok), "=r"(a)
+      "mov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, w}, h;\n\t}"
+      : "=r"(ok), "=r"(a), "=r"(b), "=r"(c)
       : "r"(src)
       : "memory");
   x = a;
+  y = b;
+  z = c;
   return ok != 0;
 }
 // tcgen05.wait::ld that the loaded registers pass through, so that no use of them moves above it.
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
 
   // One K or V tile of an item into ring stage g % STAGES, g counting the fills of all items. An
   // item's tiles in the order of their first use: K(0), K(1), V(0), K(2), V(1), .. V(n - 1).
-  auto issue_fill = [&](const PlainItem& w, int fill, int g) {
+  auto issue_fill = [&](const PlainItem& w, int kh, int vh, int fill, int g) {
     const int s = g % STAGES;
     const bool is_k = fill == 0 || ((fill & 1) != 0 && fill != 2 * w.n - 1);
     const int v = is_k ? (fill + 1) >> 1 : fill == 2 * w.n - 1 ? w.n - 1 : (fill >> 1) - 1;
@@ -244,12 +248,16 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     mbar_expect_tx(bar(B_KVFULL + s), L::TILE_BYTES);
     fills_issued[s] = g / STAGES + 1;
     const CUtensorMap* tm = is_k ? &p.tm_k : &p.tm_v;
-    const int hh = w.h / (is_k ? p.k_hdiv : p.v_hdiv);
+    const int hh = is_k ? kh : vh;
     const int bb = w.b * (is_k ? p.k_bmul : p.v_bmul);
 #pragma unroll
     for (int c = 0; c < L::CHUNKS; ++c)
       tma_load_4d(sbase + L::KV_OFF + s * L::TILE_BYTES + c * L::CHUNK_BYTES, tm,
                   bar(B_KVFULL + s), c * 64, j * BN, hh, bb);
+  };
+  auto kv_heads = [&](const PlainItem& w, int& kh, int& vh) {  // of an item
+    kh = w.h / p.k_hdiv;
+    vh = p.v_hdiv == p.k_hdiv ? kh : w.h / p.v_hdiv;
   };
   auto issue_q = [&](const PlainItem& w, int t) {
     mbar_expect_tx(bar(B_QFULL + t), L::TILE_BYTES);
@@ -306,7 +314,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     // the first copies run under the TMEM allocation and the CTA-wide sync
-    const PlainItem w = plain_item(p, blockIdx.x);
+    const PlainItem w = plain_item(p, blockIdx.x, blockIdx.y, blockIdx.z);
     if (w.n > 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_q) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_k) : "memory");
@@ -314,8 +322,10 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
 #pragma unroll
       for (int t = 0; t < ATT_NQ; ++t)
         if (w.hi[t] > w.lo[t]) issue_q(w, t);
+      int kh, vh;
+      kv_heads(w, kh, vh);
       const int first_round = min(STAGES, 2 * w.n);  // the ring is empty: nobody to wait for
-      for (int fill = 0; fill < first_round; ++fill) issue_fill(w, fill, fill);
+      for (int fill = 0; fill < first_round; ++fill) issue_fill(w, kh, vh, fill, fill);
     }
     publish(w, 0);
   }
@@ -346,6 +356,45 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     if (lane == 0) mbar_arrive(bar(B_ITEMFREE + (q & 1)));
   };
 
+  // O / l of this thread's row of Q tile t (TMEM lane) to global memory, and its log sum
+  auto store_rows = [&](int t, bool any, float l_row, float m_row, int b, int hq, int row,
+                        auto&& o_is_read) {
+    tc_fence_after();
+    const float inv = (any && l_row > 0.0f) ? __fdividef(1.0f, l_row) : 0.0f;
+    const uint32_t o_addr = (static_cast<uint32_t>((warp & 3) * 32) << 16) + O_COL + t * D;
+    uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) +
+                    2ll * (b * p.o_stride_b + static_cast<long long>(row) * p.o_stride_s +
+                           hq * p.o_stride_h);
+#pragma unroll 1
+    for (int cc = 0; cc < D; cc += 32) {
+      uint32_t orr[32];
+      if (any) {
+        tmem_ld32<0>(o_addr + cc, orr);
+        tmem_wait_ld32<0>(orr);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) orr[e] = 0u;
+      }
+      if (cc == D - 32) o_is_read();
+      if (row < p.Sq) {
+#pragma unroll
+        for (int e = 0; e < 32; e += 8) {
+          uint4 v;
+          uint32_t* vv = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            vv[i] = pack16<BF16>(__uint_as_float(orr[e + 2 * i]) * inv,
+                                 __uint_as_float(orr[e + 2 * i + 1]) * inv);
+          *reinterpret_cast<uint4*>(orow + 2 * (cc + e)) = v;
+        }
+      }
+      __syncwarp();
+    }
+    if (p.lse && row < p.Sq)
+      p.lse[b * p.lse_stride_b + hq * p.lse_stride_h + row] =
+          (any && l_row > 0.0f) ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+  };
+
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::OTHER));
     if (warp == 12) {
@@ -354,7 +403,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         auto wait = [&](int i, uint32_t parity) {
           return mbar_wait(bar(i), parity, abort_flag, p.status, ATT_ST_PRODUCER);
         };
-        PlainItem w = plain_item(p, blockIdx.x);
+        PlainItem w = plain_item(p, blockIdx.x, blockIdx.y, blockIdx.z);
+        int kh, vh;
+        kv_heads(w, kh, vh);
         int base = 0;                        // fills of the items before this one
         int start = min(STAGES, 2 * w.n);    // of this one, issued before the CTA-wide sync
         bool ok = true, asked = false;
@@ -362,7 +413,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         auto fill_one = [&](int fill) {
           const int g = base + fill;
           if (g >= STAGES) ok = wait(B_KVEMPTY + g % STAGES, ((g / STAGES) & 1) ^ 1);
-          if (ok) issue_fill(w, fill, g);
+          if (ok) issue_fill(w, kh, vh, fill, g);
         };
 #pragma unroll 1
         while (true) {
@@ -372,6 +423,11 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           base += total;
           start = 0;
           if (!ok) break;
+          if (p.single) {  // there is no other item
+            w.valid = 0;
+            publish(w, 1);
+            break;
+          }
           // The next item is asked for when this one's last tiles have been: some visits before its
           // end, enough to hide the answer; earlier would take items from CTAs that are done sooner.
           mbar_expect_tx(bar(B_NEXT), 16);
@@ -380,11 +436,15 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           ok = wait(B_NEXT, q & 1);
           if (!ok) break;
           asked = false;
-          int idx;
-          const bool more = requested_block(sbase + L::NEXT_OFF, idx);
+          int x, y, z;
+          const bool more = requested_block(sbase + L::NEXT_OFF, x, y, z);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          if (more) w = plain_item(p, idx);
-          else w.valid = 0;
+          if (more) {
+            w = plain_item(p, x, y, z);
+            kv_heads(w, kh, vh);
+          } else {
+            w.valid = 0;
+          }
           ++q;
           if (q >= 2) ok = wait(B_ITEMFREE + (q & 1), ((q >> 1) & 1) ^ 1);
           if (!ok) break;
@@ -488,9 +548,11 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       auto free_fill = [&](int f) {  // once this warp's MMAs are done with it
         if (ok && elect_one()) tc_commit(bar(B_KVEMPTY + (f & (STAGES - 1))));
       };
-      // Whether a barrier's phase is complete, without waiting for it.
+      // Whether a barrier's phase is complete, without waiting for it (try_wait would be suspended for
+      // microseconds where only this warp's next step can complete it: 2 x 6000 full, 12 heads x 64,
+      // whose last Q tile is empty, 547 us, now 307).
       auto ready = [&](int b, uint32_t parity) -> bool {
-        return __all_sync(0xffffffffu, mbar_try_wait(bar(b), parity));
+        return __all_sync(0xffffffffu, mbar_test(bar(b), parity));
       };
       // Values that are the same in every lane, in a way the compiler knows.
       auto uniform = [](int x) { return __reduce_max_sync(0xffffffffu, x); };
@@ -631,50 +693,16 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           opar[t] ^= 1u;
         }
         if (!ok) break;
-        tc_fence_after();
         const float* stat = reinterpret_cast<const float*>(smem + L::STAT_OFF) + t * 2 * ATT_BM;
-        const float l_row = stat[r], m_row = stat[ATT_BM + r];
-        const float inv = (any && l_row > 0.0f) ? __fdividef(1.0f, l_row) : 0.0f;
-        const int row = w.m0 + t * t_rows + r, hq = w.h + t * t_head;
-        const uint32_t o_addr = (static_cast<uint32_t>(wq * 32) << 16) + O_COL + t * D;
-        uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) +
-                        2ll * (w.b * p.o_stride_b + static_cast<long long>(row) * p.o_stride_s +
-                               hq * p.o_stride_h);
-#pragma unroll 1
-        for (int cc = 0; cc < D; cc += 32) {
-          uint32_t orr[32];
-          if (any) {
-            tmem_ld32<0>(o_addr + cc, orr);
-            tmem_wait_ld32<0>(orr);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) orr[e] = 0u;
-          }
-          if (cc == D - 32) {  // O and the statistics are read: the next item may write them
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              if (any) mbar_arrive(bar(B_OFREE + t));
-              mbar_arrive(bar(B_STATFREE + t));
-            }
-          }
-          if (row < p.Sq) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 v;
-              uint32_t* vv = reinterpret_cast<uint32_t*>(&v);
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                vv[i] = pack16<BF16>(__uint_as_float(orr[e + 2 * i]) * inv,
-                                     __uint_as_float(orr[e + 2 * i + 1]) * inv);
-              *reinterpret_cast<uint4*>(orow + 2 * (cc + e)) = v;
-            }
-          }
-          __syncwarp();
-        }
-        if (p.lse && row < p.Sq)
-          p.lse[w.b * p.lse_stride_b + hq * p.lse_stride_h + row] =
-              (any && l_row > 0.0f) ? (m_row + log2f(l_row)) * 0.6931471805599453f : -INFINITY;
+        store_rows(t, any, stat[r], stat[ATT_BM + r], w.b, w.h + t * t_head, w.m0 + t * t_rows + r,
+                   [&] {  // O and the statistics are read: the next item may write them
+                     tc_fence_before();
+                     __syncwarp();
+                     if (lane == 0) {
+                       if (any) mbar_arrive(bar(B_OFREE + t));
+                       mbar_arrive(bar(B_STATFREE + t));
+                     }
+                   });
       }
       return ok;
     };
@@ -691,7 +719,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       it.any0 = w.hi[0] > w.lo[0];
       it.any1 = w.hi[1] > w.lo[1];
       item_read(q);
-      if (!valid || !finish(it)) break;
+      if (!valid || p.single || !finish(it)) break;  // a single item's rows are the softmax warps'
     }
   } else {
     // =========================== softmax ==============================================
@@ -721,6 +749,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       float slope2 = 0.0f;
       if (BIAS != AP_NONE && valid && p.slopes)
         slope2 = p.slopes[w.h + t * t_head] * 1.4426950408889634f;
+      const int ib = w.b, ihq = w.h + t * t_head;
       item_read(q);
       if (!valid) break;
       const int row1 = min(p.Sq, row0 + ATT_BM) - 1;
@@ -855,6 +884,14 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         l_run += sum[0].x + sum[0].y;
       }
       if (!ok) break;
+      if (p.single) {
+        // No next item to start on: these warps write their rows themselves, both Q tiles at once and
+        // without the hand-over (8 x 128 keys, 16 heads x 64: 7.9 us with the epilogue warps and a
+        // request for a next item, 7.1 so).
+        if (n_it > 0) ok = wait(B_ODONE + t, 0);
+        if (ok) store_rows(t, n_it > 0, l_run, m_run, ib, ihq, row, [] {});
+        break;
+      }
       if (q > 0) {
         ok = wait(B_STATFREE + t, (q - 1) & 1);  // the last item's statistics have been read
         if (!ok) break;
@@ -913,10 +950,10 @@ static int launch_plain(const AttnParams& p, cudaStream_t stream) {
       return TRX_ERR_CUDA;
     if (cacheable) configured[dev].store(true, std::memory_order_release);
   }
-  const int64_t items = static_cast<int64_t>(p.m_blocks) * p.slots;
-  if (items > 0x7fffffff) return TRX_ERR_SHAPE;
-  attn_plain_kernel<D, BF16, BIAS>
-      <<<static_cast<unsigned>(items), AP_THREADS, PlainSmem<D>::DYN_BYTES, stream>>>(p);
+  const int rows = p.pair_heads ? ATT_BM : ATT_NQ * ATT_BM;
+  const unsigned m = (p.Sq + rows - 1) / rows, h = p.pair_heads ? p.Hq / 2 : p.Hq, b = p.B;
+  const dim3 grid = p.order == AP_MHB ? dim3(m, h, b) : p.order == AP_HMB ? dim3(h, m, b) : dim3(h, b, m);
+  attn_plain_kernel<D, BF16, BIAS><<<grid, AP_THREADS, PlainSmem<D>::DYN_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? TRX_OK : TRX_ERR_CUDA;
 }
 
@@ -931,17 +968,15 @@ static int launch_plain_bias(const AttnParams& p, cudaStream_t stream) {
 
 int launch_attn_plain(AttnParams& p, int64_t D, cudaStream_t stream) {
   const int rows = p.pair_heads ? ATT_BM : ATT_NQ * ATT_BM;
-  p.m_blocks = (p.Sq + rows - 1) / rows;
-  p.slots = p.B * (p.pair_heads ? p.Hq / 2 : p.Hq);
-  p.slot_group = 1;
-  if (p.causal) {
-    // The heaviest row blocks of a group of slots first, so that the CTAs end together (one slot
-    // after the other, 2 x 4096 x 32 / 8 heads: 283 us, so 255); as many slots to a group as have
-    // their keys and values in a third of L2.
-    const double kv = 4.0 * p.Sk * static_cast<double>(D);
-    const int share = max(1, p.group / (p.pair_heads ? 2 : 1));  // slots per kv head
-    const double fit = 40e6 / max(kv, 1.0) * share;
-    p.slot_group = fit >= p.slots ? p.slots : fit < 1.0 ? 1 : static_cast<int>(fit);
+  const int64_t m = (p.Sq + rows - 1) / rows, h = p.pair_heads ? p.Hq / 2 : p.Hq;
+  p.single = m * h * p.B <= sm_count_of_current_device() ? 1 : 0;
+  p.order = AP_MHB;
+  if (p.causal && m <= 65535) {
+    // Heaviest row blocks first (one head after the other, 2 x 4096 x 32 / 8 heads: 283 us, so 255),
+    // over all heads whose keys and values fit a third of L2, or those of one batch.
+    const double kv = 4.0 * p.Sk * static_cast<double>(D) * p.Hq / p.group;  // bytes of a batch
+    if (kv * p.B <= 40e6) p.order = AP_HBM;
+    else if (kv <= 100e6) p.order = AP_HMB;
   }
   if (D == 128)
     return p.is_bf16 ? launch_plain_bias<128, true>(p, stream) : launch_plain_bias<128, false>(p, stream);
