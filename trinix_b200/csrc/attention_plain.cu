@@ -25,7 +25,7 @@
 //   * the issuing warps stay converged and elect a lane, and every branch goes by a vote: descriptors
 //     are then uniform registers (from one lane in divergent code 4 x 4096 full: 1142 us, so 991);
 //   * one issuing warp per Q tile: a wait on a ready barrier costs such a warp some 200 cycles, and
-//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1874;
+//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1904, with its registers 1874 to 1910;
 //     window 1024: 1304, 1097; 8 x 2048 causal, 16 heads x 64: 188, 137);
 //   * cut tiles: one uniform test per visit, then bit masks (2900 -> 600 cycles for such a tile).
 // Measured and not taken: S shared by both tiles with P beside it (1016-1200 us on 4 x 4096 full
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           base += total;
           start = 0;
           if (!ok) break;
-          if (p.single) {  // there is no other item
+          if (p.single) {  // no other item, and no answer to wait for (8 x 128 keys, 16 heads x 64: 7.9 us, so 7.1)
             w.valid = 0;
             publish(w, 1);
             break;
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       it.any0 = w.hi[0] > w.lo[0];
       it.any1 = w.hi[1] > w.lo[1];
       item_read(q);
-      if (!valid || p.single || !finish(it)) break;  // a single item's rows are the softmax warps'
+      if (!valid || !finish(it)) break;
     }
   } else {
     // =========================== softmax ==============================================
@@ -749,7 +749,6 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       float slope2 = 0.0f;
       if (BIAS != AP_NONE && valid && p.slopes)
         slope2 = p.slopes[w.h + t * t_head] * 1.4426950408889634f;
-      const int ib = w.b, ihq = w.h + t * t_head;
       item_read(q);
       if (!valid) break;
       const int row1 = min(p.Sq, row0 + ATT_BM) - 1;
@@ -884,14 +883,6 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         l_run += sum[0].x + sum[0].y;
       }
       if (!ok) break;
-      if (p.single) {
-        // No next item to start on: these warps write their rows themselves, both Q tiles at once and
-        // without the hand-over (8 x 128 keys, 16 heads x 64: 7.9 us with the epilogue warps and a
-        // request for a next item, 7.1 so).
-        if (n_it > 0) ok = wait(B_ODONE + t, 0);
-        if (ok) store_rows(t, n_it > 0, l_run, m_run, ib, ihq, row, [] {});
-        break;
-      }
       if (q > 0) {
         ok = wait(B_STATFREE + t, (q - 1) & 1);  // the last item's statistics have been read
         if (!ok) break;
