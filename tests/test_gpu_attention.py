@@ -2,6 +2,7 @@
 attention), through triton_attn_func / the C ABI. Tolerance from the project baseline:
 2e-2 max abs error in bf16."""
 import ctypes
+import math
 import threading
 
 import pytest
@@ -534,6 +535,29 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     ref_lse = torch.logsumexp(s, -1).reshape(B, Hq, Sq)
     # sums of up to 33000 fp32 terms in another order: below 33000 * 2^-24 of the sum
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
+
+
+@pytest.mark.parametrize("Sq", [17, 300])
+@pytest.mark.parametrize("Sk", [128, 1024])
+def test_row_sums_lose_no_more_than_chains_of_sixteen(cuda, Sq, Sk):
+    """One key of weight 1 in the first eight columns, 2^-25 for every other: in fp32 those that are
+    added behind the 1 in its chain are lost, and nothing else is. A row of a tile is summed in eight
+    chains of 16, so 15 are; with a chain of 32 it would be 31."""
+    from trinix_b200 import ops
+    B, D = 8, 128
+    q = torch.zeros(B, Sq, 2, D)
+    q[..., 0] = 1.0
+    k = torch.zeros(B, Sk, 2, D)
+    k[..., 0] = -25.0
+    for b in range(B):
+        k[b, b, :, 0] = 0.0
+    v = torch.zeros(B, Sk, 2, D)
+    q, k, v = (t.bfloat16().to(cuda) for t in (q, k, v))
+    # the score in the log2 domain is q.k to 1e-7, the weights 2^-25 (1 +- 3e-6)
+    _, lse = ops.attention(q, k, v, scale=math.log(2.0), return_lse=True)
+    exact = math.log1p((Sk - 1) * 2.0 ** -25)
+    # one more of them for the last roundings, and the weights' own error
+    assert float((lse.double() - exact).abs().max()) <= 16 * 2.0 ** -25 + Sk * 2.0 ** -25 * 3e-6
 
 
 @pytest.mark.parametrize("B,Sq,Sk,Hq,Hk,D,causal,window,alibi,scale", [

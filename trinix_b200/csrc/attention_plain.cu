@@ -769,7 +769,13 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       }
       const float unit = BIAS == AP_GENERAL ? 1.0f : sl2;
       const float kc = BIAS == AP_RAMP ? __fdividef(slope2, sl2) : 0.0f;
-      float m_run = -INFINITY, l_run = 0.0f;
+      // The row sum in four shares, one of every fourth pair of columns; in a tile each is a chain of
+      // the 16 even and one of the 16 odd columns. The order of attention.cu, whose rows are held by
+      // four threads, so that the two agree to the last bit. Two chains and one share, 2 to 3 us in 200
+      // faster with ALiBi or a window (16 x 4096: 2288 / 2333 us, 4 x 3001 190.6 / 193.4; causal 2132 /
+      // 2119), leave a relative error of 1.4 / 2.0 x 2^-24 (rms, 4096 / 8192 keys), these 0.9 / 1.1.
+      float m_run = -INFINITY;
+      float2 l_run[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
       float m_ref = 0.0f;  // m_run, or 0 while no key has been visible
 
 #pragma unroll 1
@@ -840,7 +846,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         if (__any_sync(0xffffffffu, grown)) {
           const float factor = grown ? fast_exp2(m_run - m_tile) : 1.0f;  // 0 when m_run == -inf
           if (grown) m_run = m_ref = m_tile;
-          l_run *= factor;
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            l_run[i] = make_float2(l_run[i].x * factor, l_run[i].y * factor);
           if (itn > 0) {
 #pragma unroll 1
             for (int cc = 0; cc < D; cc += 32) {
@@ -859,7 +867,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         // P = exp2(x - m), 32 keys (16 packed columns) at a time, over the scores
         static_assert(AP_REST == 2, "the last 32 keys are two MMAs");
         const float2 unit2 = make_float2(unit, unit), neg2 = make_float2(neg, neg);
-        float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+        float2 sum[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[i] = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int g = 0; g < BN / 32; ++g) {
           uint32_t pk[16];
@@ -868,7 +878,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             const int c = 32 * g + 2 * i;
             const float2 x = fma2(pair_of(sr + c), unit2, neg2);
             const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-            sum[i & 1] = add2(sum[i & 1], e);
+            sum[i & 3] = add2(sum[i & 3], e);
             pk[i] = pack16<BF16>(e.x, e.y);
           }
           tmem_st16(s_addr + 16 * g, pk);
@@ -879,15 +889,17 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             if (lane == 0) mbar_arrive(bar((g == BN / 32 - 1 ? B_PREST : B_PFULL) + t));
           }
         }
-        sum[0] = add2(sum[0], sum[1]);
-        l_run += sum[0].x + sum[0].y;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          l_run[i] = add2(l_run[i], make_float2(sum[2 * i].x + sum[2 * i].y,
+                                                sum[2 * i + 1].x + sum[2 * i + 1].y));
       }
       if (!ok) break;
       if (q > 0) {
         ok = wait(B_STATFREE + t, (q - 1) & 1);  // the last item's statistics have been read
         if (!ok) break;
       }
-      stat[rl] = l_run;
+      stat[rl] = (l_run[0].x + l_run[0].y) + (l_run[1].x + l_run[1].y);
       stat[ATT_BM + rl] = m_run;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(B_STAT + t));
