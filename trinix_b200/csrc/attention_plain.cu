@@ -33,11 +33,11 @@
 // memory, 48 cycles instead of 32), exponentials of the two tiles in forced turns (2064).
 // Every wait is bounded, see attention_common.cuh.
 #include "attention_common.cuh"
+#include "attention_issue.cuh"
 
 namespace trx {
 
 constexpr int AP_THREADS = 512;
-constexpr int AP_STAGES = 4;  // K / V ring
 // P is handed over in two pieces: the P V of the first 96 keys runs while the last 32 are
 // exponentiated (causal 16 x 4096: 1994 us in one piece, 1904 so, 2064 in halves).
 constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
@@ -473,11 +473,11 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       // One warp per Q tile, each between its softmax warps and the tensor pipe: every cycle it spends
       // between two groups of MMAs is one in which that tile's chain stands still. The warp stays
       // converged and one elected lane issues, so that addresses and descriptors are uniform
-      // registers; a run of visits with nothing special has a loop of its own.
+      // registers; a run of visits with nothing special has a loop of its own. The order of the work is
+      // plain_issue's (attention_issue.cuh); here is what its steps are.
       const int t = warp - 13;
       const uint32_t idesc_qk = make_idesc(BF16 ? 1 : 0, ATT_BM, BN, 0, 0);
       const uint32_t idesc_pv = make_idesc(BF16 ? 1 : 0, ATT_BM, D, 0, 1);
-      static_assert((STAGES & (STAGES - 1)) == 0, "ring depth must be a power of two");
       // Descriptors differ only in their 14-bit start-address field (address >> 4), the low part
       // of the low word.
       const uint64_t desc_k_major = make_desc(0, 16, 1024);               // K-major, SBO 1 KB
@@ -494,18 +494,13 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       auto wait = [&](int b, uint32_t parity) {
         return mbar_wait_warp<false>(bar(b), parity, abort_flag, p.status, ATT_ST_MMA);
       };
-      bool ok = true;
-      uint32_t ppar = 0, qpar = 0;  // parity of the next P and of the next Q tile
-      bool s_busy = false;          // a Q K^T is issued whose P V is not
-      uint32_t keyed = 0;           // items with keys whose P V have begun
-      int kf = 0, vf = 0;           // ring fill of the next Q K^T and of the next P V
+      uint32_t ppar = 0;  // parity of the next P
       const uint32_t d_o = O_COL + t * D, d_s = S_COL + t * BN, qst = q_lo + t * T16;
 
       // O_t += P_t V (P from TMEM, V MN-major from its ring stage); `acc` = 0 clears O first
-      auto pv = [&](uint32_t acc) {
+      auto pv = [&](int vf, uint32_t acc) -> bool {
         const uint32_t vst = v_lo + (static_cast<uint32_t>(vf) & (STAGES - 1)) * T16;
-        ok = wait(B_PFULL + t, ppar);
-        if (!ok) return;
+        if (!wait(B_PFULL + t, ppar)) return false;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -513,21 +508,20 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             mma_ts(d_o, d_s + kk * 8, desc_of(vst + kk * (2048 >> 4), dv_hi), idesc_pv,
                    kk == 0 ? acc : 1u);
         }
-        ok = wait(B_PREST + t, ppar);
+        const bool rest = wait(B_PREST + t, ppar);
         ppar ^= 1u;
-        s_busy = false;
-        if (!ok) return;
+        if (!rest) return false;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
           for (int kk = BN / 16 - AP_REST; kk < BN / 16; ++kk)
             mma_ts(d_o, d_s + kk * 8, desc_of(vst + kk * (2048 >> 4), dv_hi), idesc_pv, 1u);
         }
+        return true;
       };
       // S = Q_t K^T (both operands K-major in shared memory), then announce it to the softmax warps.
       // The P V that reads the P in its columns is ahead of it in the pipe.
-      auto qk = [&]() {
-        s_busy = true;
+      auto qk = [&](int kf) {
         tc_fence_after();
         const uint32_t kst = k_lo + (static_cast<uint32_t>(kf) & (STAGES - 1)) * T16;
         if (elect_one()) {
@@ -542,11 +536,8 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           tc_commit(bar(B_SFULL + t));
         }
       };
-      auto wait_fill = [&](int f) {
-        if (ok) ok = wait(B_KVFULL + (f & (STAGES - 1)), (f / STAGES) & 1);
-      };
-      auto free_fill = [&](int f) {  // once this warp's MMAs are done with it
-        if (ok && elect_one()) tc_commit(bar(B_KVEMPTY + (f & (STAGES - 1))));
+      auto commit = [&](int b) {  // once this warp's MMAs are done
+        if (elect_one()) tc_commit(bar(b));
       };
       // Whether a barrier's phase is complete, without waiting for it (try_wait would be suspended for
       // microseconds where only this warp's next step can complete it: 2 x 6000 full, 12 heads x 64,
@@ -556,15 +547,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       };
       // Values that are the same in every lane, in a way the compiler knows.
       auto uniform = [](int x) { return __reduce_max_sync(0xffffffffu, x); };
-
-      // The work is the sequence of this Q tile's visits over all items. The Q K^T run one visit
-      // ahead of the P V, into the next item too:  .. P V(v), Q K(v + 1), P V(v + 1) ..
-      // The K and V tiles of visits without this Q tile are only released. Nothing ahead of a
-      // pending P V is waited for: the ring may be held up by a V tile that this P V frees.
-      struct Cursor {
-        int lo, hi, n, item, v;
-      };
-      auto open = [&](Cursor& c, int item) -> bool {  // false: there is no such item
+      auto open = [&](PlainCursor& c, int item, bool& ok) -> bool {  // false: there is no such item
         ok = wait(B_ITEM + (item & 1), (item >> 1) & 1);
         if (!ok) return false;
         volatile PlainItem& w = items[item & 1];
@@ -579,88 +562,20 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         item_read(item);
         return valid;
       };
-      auto step_qk = [&](Cursor& c) {
-        const int v = c.v;
-        wait_fill(kf);
-        if (ok && v == c.lo && c.lo < c.hi) {
-          ok = wait(B_QFULL + t, qpar);
-          qpar ^= 1u;
-        }
-        if (ok && v >= c.lo && v < c.hi) qk();
-        if (ok && v == c.hi - 1 && c.lo < c.hi && elect_one()) tc_commit(bar(B_QEMPTY + t));
-        free_fill(kf);
-        kf += v == 0 && c.n > 1 ? 1 : 2;
-        if (v + 1 == c.n) kf += c.n > 1 ? 1 : 0;
-        c.v = v + 1;
-      };
-      auto step_pv = [&](Cursor& c) {
-        const int v = c.v;
-        wait_fill(vf);
-        if (ok && v >= c.lo && v < c.hi) {
-          // the epilogue is done with the last O (items without keys have none: it does not wait
-          // for this warp there, so they must not count)
-          if (v == c.lo && keyed++ > 0) ok = wait(B_OFREE + t, keyed & 1);
-          if (ok) pv(v == c.lo ? 0u : 1u);
-          if (ok && v == c.hi - 1 && elect_one()) tc_commit(bar(B_ODONE + t));
-        }
-        free_fill(vf);
-        vf += v + 2 >= c.n ? 1 : 2;
-        c.v = v + 1;
-      };
-
-      Cursor qc, pc, nc;  // of the Q K^T, of the P V, and the next item's
-      bool more = open(qc, 0);  // there may be another item
-      pc = qc;
-      vf = qc.n > 1 ? 2 : qc.n;  // V(0) comes behind K(1) of its item, if there is one
-      bool known = false;        // nc is the item after pc's
-#pragma unroll 1
-      while (ok) {
-        while (ok) {
-          const bool behind = qc.item != pc.item || qc.v > pc.v;  // there is a P V step to take
-          if (qc.v == qc.n) {
-            if (qc.item > pc.item || !more) break;  // at the end of what it may go to
-            const int i = qc.item + 1;
-            if (pc.v < pc.n && !ready(B_ITEM + (i & 1), (i >> 1) & 1)) break;
-            more = open(nc, i);
-            if (!more) break;
-            known = true;
-            qc = nc;
-            continue;
-          }
-          if (s_busy) break;
-          if (behind && !ready(B_KVFULL + (kf & (STAGES - 1)), (kf / STAGES) & 1)) break;
-          if (behind && qc.v == qc.lo && !ready(B_QFULL + t, qpar)) break;
-          step_qk(qc);
-        }
-        if (!ok) break;
-        if (qc.item == pc.item && qc.v == pc.v + 1 && s_busy && pc.v > pc.lo) {
-          const int last = pc.hi - 3;  // of the P V visits
-#pragma unroll 1
-          while (pc.v <= last) {
-            wait_fill(vf);
-            wait_fill(kf);
-            if (ok) pv(1u);
-            free_fill(vf);
-            if (ok) qk();
-            free_fill(kf);
-            if (!ok) break;
-            kf += 2;
-            vf += 2;
-            ++pc.v;
-            ++qc.v;
-          }
-          if (!ok) break;
-        }
-        if (pc.v == pc.n) {
-          // on to the next item, if there is one
-          if (!known) break;
-          pc = nc;
-          known = false;
-          vf += pc.n > 1 ? 2 : pc.n;
-          continue;
-        }
-        if (pc.item != qc.item || pc.v < qc.v) step_pv(pc);
-      }
+      PlainSteps steps{
+          open,
+          [&](int i) { return ready(B_ITEM + (i & 1), (i >> 1) & 1); },
+          [&](int f) { return wait(B_KVFULL + (f & (STAGES - 1)), (f / STAGES) & 1); },
+          [&](int f) { return ready(B_KVFULL + (f & (STAGES - 1)), (f / STAGES) & 1); },
+          [&](int f) { commit(B_KVEMPTY + (f & (STAGES - 1))); },
+          [&](uint32_t parity) { return wait(B_QFULL + t, parity); },
+          [&](uint32_t parity) { return ready(B_QFULL + t, parity); },
+          qk,
+          [&] { commit(B_QEMPTY + t); },
+          [&](uint32_t parity) { return wait(B_OFREE + t, parity); },
+          pv,
+          [&] { commit(B_ODONE + t); }};
+      const bool ok = plain_issue(steps);
       if (!ok && lane == 0) {
         // drain whatever was issued before giving up
         tc_commit(bar(B_DRAIN + t));
