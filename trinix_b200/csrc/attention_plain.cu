@@ -576,8 +576,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
           pv,
           [&] { commit(B_ODONE + t); }};
       const bool ok = plain_issue(steps);
-      if (!ok && lane == 0) {
-        // drain whatever was issued before giving up
+      if (!ok && elect_one()) {
+        // drain whatever was issued before giving up: a commit follows the MMAs of its own thread, and
+        // which lane elect.sync takes is not specified
         tc_commit(bar(B_DRAIN + t));
         const uint64_t t0 = global_ns();
         while (!mbar_try_wait(bar(B_DRAIN + t), 0) && global_ns() - t0 < ATT_WAIT_NS) {
