@@ -537,6 +537,26 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("Sq", [128, 256])  # an empty second Q tile, and two
+def test_one_item_of_half_a_million_key_tiles(cuda, Sq):
+    """2^26 keys in one work item: 2^19 visits of a microsecond or more, which is longer than the 400 ms
+    after which a wait gives up. Keys of zeros and values of ones, so every sum is exact in fp32: the
+    row sum 2^26 in shares of 2^24, O in steps of 16."""
+    from trinix_b200 import ops
+    Sk, D = 1 << 26, 64
+    if torch.cuda.mem_get_info()[0] < 20 << 30:
+        pytest.skip("needs 20 GB")
+    q = torch.ones(1, Sq, 1, D, device=cuda, dtype=torch.bfloat16)
+    k = torch.zeros(1, Sk, 1, D, device=cuda, dtype=torch.bfloat16)
+    v = torch.ones(1, Sk, 1, D, device=cuda, dtype=torch.bfloat16)
+    out, lse = ops.attention(q, k, v, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    assert bool((out == 1).all())
+    assert float((lse - 26 * math.log(2.0)).abs().max()) <= 4e-6  # 18.0 to an fp32 ulp or two
+    del k, v
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("Sq", [17, 300])
 @pytest.mark.parametrize("Sk", [128, 1024])
 def test_row_sums_lose_no_more_than_chains_of_sixteen(cuda, Sq, Sk):

@@ -184,6 +184,47 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __any_sync(0xffffffffu, mbar_poll_warp_call(bar, parity, abort_flag, status, code));
 }
+// A wait for something that takes as long as a whole work item (its row statistics, the next item): an
+// item may have any number of KV tiles, so the time counts from the last `progress` of the CTA.
+__device__ __forceinline__ bool mbar_poll_item(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code, volatile int* progress) {
+  uint64_t t0 = 0;
+  int seen = 0;
+#pragma unroll 1
+  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 63u) == 63u) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      const int now = *progress;
+      if (__any_sync(0xffffffffu, t0 == 0 || now != seen)) {
+        seen = now;
+        t0 = global_ns();
+        i = 0;
+      } else if (__any_sync(0xffffffffu, global_ns() - t0 > ATT_WAIT_NS)) {
+        break;
+      }
+    }
+  }
+  *abort_flag = 1;
+  atomicOr(status, code);
+  return false;
+}
+static __device__ __noinline__ bool mbar_poll_item_call(uint32_t bar, uint32_t parity,
+                                                        volatile int* abort_flag,
+                                                        unsigned int* status, unsigned code,
+                                                        volatile int* progress) {
+  return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
+}
+template <bool INLINE>
+__device__ __forceinline__ bool mbar_wait_item(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code, volatile int* progress) {
+  if constexpr (INLINE) return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __any_sync(0xffffffffu,
+                    mbar_poll_item_call(bar, parity, abort_flag, status, code, progress));
+}
 // One lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
   uint32_t is;

@@ -350,6 +350,11 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
                    : "memory");
     return;
   }
+  // What takes as long as a work item is waited for while the ring is being filled.
+  auto wait_item = [&](auto inline_tag, int i, uint32_t parity) -> bool {
+    return mbar_wait_item<decltype(inline_tag)::value>(bar(i), parity, abort_flag, p.status,
+                                                       ATT_ST_SOFTMAX, fills_issued);
+  };
   // an item has been read: a warp's arrival
   auto item_read = [&](int q) {
     __syncwarp();
@@ -603,7 +608,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
 #pragma unroll
       for (int t = 0; t < ATT_NQ; ++t) {
         const bool any = t ? w.any1 : w.any0;
-        if (ok) ok = wait(B_STAT + t, w.q & 1);
+        if (ok) ok = wait_item(std::false_type{}, B_STAT + t, w.q & 1);
         if (ok && any) {
           ok = wait(B_ODONE + t, opar[t]);
           opar[t] ^= 1u;
@@ -624,7 +629,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     };
 #pragma unroll 1
     for (int q = 0;; ++q) {
-      if (!wait(B_ITEM + (q & 1), (q >> 1) & 1)) break;
+      if (!wait_item(std::false_type{}, B_ITEM + (q & 1), (q >> 1) & 1)) break;
       volatile PlainItem& w = items[q & 1];
       const bool valid = w.valid != 0;
       Item it;
@@ -655,7 +660,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     };
 #pragma unroll 1
     for (int q = 0;; ++q) {
-      ok = wait(B_ITEM + (q & 1), (q >> 1) & 1);
+      ok = wait_item(std::true_type{}, B_ITEM + (q & 1), (q >> 1) & 1);
       if (!ok) break;
       volatile PlainItem& w = items[q & 1];
       const bool valid = w.valid != 0;
