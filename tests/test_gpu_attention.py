@@ -537,6 +537,32 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("extra", [0, 1])  # one work item per SM, and one more
+@pytest.mark.parametrize("causal,alibi", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("Sq,Sk,D", [(17, 1, 128), (130, 128, 64), (256, 129, 128), (200, 700, 128)])
+def test_one_item_per_sm(cuda, Sq, Sk, D, causal, alibi, extra):
+    """Launches of one work item per SM have kernels of their own; one item more takes the others.
+    Reference in fp32 on the device, bounds as in test_more_work_items_than_ctas."""
+    from trinix_b200 import ops
+    H = torch.cuda.get_device_properties(cuda).multi_processor_count + extra
+    q, k, v = (t.to(cuda) for t in _qkv(1, Sq, Sk, H, H, D, seed=Sq + Sk))
+    slopes = torch.linspace(0.01, 0.5, H, device=cuda) if alibi else None
+    out, lse = ops.attention(q, k, v, causal=causal, alibi_slopes=slopes, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    s = torch.einsum("bihd,bjhd->bhij", q.float(), k.float()) * D ** -0.5
+    i, j = torch.arange(Sq, device=cuda)[:, None], torch.arange(Sk, device=cuda)[None]
+    if alibi:
+        s = s - slopes.view(1, -1, 1, 1) * (i - j).abs()
+    if causal:
+        s = s.masked_fill(j > i, float("-inf"))
+    largest = max(1.0, float(s[~torch.isinf(s)].abs().max()))
+    assert float((lse - torch.logsumexp(s, -1)).abs().max()) <= 1e-5 * (5 + largest)
+    p = torch.softmax(s, -1)
+    ref = torch.einsum("bhij,bjhd->bihd", p, v.float())
+    bound = 2.0 ** -8 * (ref.abs() + torch.einsum("bhij,bjhd->bihd", p, v.float().abs())) + 1e-4
+    assert bool(((out.float() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("Sq", [128, 256])  # an empty second Q tile, and two
 def test_one_item_of_half_a_million_key_tiles(cuda, Sq):
     """2^26 keys in one work item: 2^19 visits of a microsecond or more, which is longer than the 400 ms

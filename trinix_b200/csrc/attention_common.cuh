@@ -54,9 +54,8 @@ struct AttnParams {
   int reverse_kv;      // visit a row block's KV tiles from the last to the first
   int pair_heads;      // the two Q tiles of a CTA: same 128 rows of two query heads that share a
                        // kv head (1), or two consecutive 128-row blocks of one head (0)
-  // attention_plain.cu: which grid dimension counts row blocks, heads (or pairs) and batches; no more
-  // CTAs than SMs, so that each has one work item
-  int order, single;
+  int order;           // attention_plain.cu: which grid dimension counts row blocks, heads (or
+                       // pairs) and batches
   // dense additive mask (B, Hq, Sq, Sk) with unit key stride; batch / head strides may be 0
   const void* bias;
   long long bias_sb, bias_sh, bias_sq;  // elements
