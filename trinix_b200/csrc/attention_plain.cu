@@ -41,6 +41,14 @@ constexpr int AP_THREADS = 512;
 // P is handed over in two pieces: the P V of the first 96 keys runs while the last 32 are
 // exponentiated (causal 16 x 4096: 1994 us in one piece, 1904 so, 2064 in halves).
 constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
+// Cycles by which Q tile 1's first softmax waits in a launch of one item per CTA. Both Q tiles' first
+// scores are ready at the same time, and tiles in step stay so: both wait for the special-function
+// unit, then both for the tensor pipe, 2.3 us a visit instead of 1.6 (512 queries x 8192 keys, 32 / 8
+// heads x 128: 152 us, so 108; x 4096 84, 58; 1 x 1000 27.3, 22.0; 2 x 256 12.1, 11.1; a window of
+// 256 on 1024 15.6, 15.2). 1000 / 1250 / 1750 cycles: 109.3 / 108.5 / 108.7, 1 x 1000 25.4 / 22.9 /
+// 21.8, 2 x 256 11.5 / 11.2 / 11.2. The same in launches of several items per CTA gained 1 to 3 % on
+// some and lost as much on others. A single visit (up to 128 keys) has nobody to get out of step with.
+constexpr unsigned AP_LAG = 1500;
 
 // What is added to the scaled scores: nothing; ALiBi as one ramp per row (every visible key at or
 // before its query); ALiBi on either side of the query, or a scale that is not positive.
@@ -705,6 +713,13 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         ok = wait(B_SFULL + t, s_par);
         if (!ok) break;
         s_par ^= 1u;
+        if (SINGLE && t == 1 && itn == 0 && n_it > 1) {
+          // half a visit behind the other Q tile, see AP_LAG
+          const unsigned begin = static_cast<unsigned>(clock());
+          for (int i = 0; i < 4096 && static_cast<unsigned>(clock()) - begin < AP_LAG; ++i) {
+          }
+          __syncwarp();
+        }
         tc_fence_after();
         // by a vote: a branch that the compiler knows to be uniform
         const bool cut = __any_sync(0xffffffffu, c0 + BN - 1 > hi_min || c0 < lo_max);
