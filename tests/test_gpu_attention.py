@@ -537,6 +537,41 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("B,Sq,Sk,H,D,window,dtype", [
+    (1, 256, 256, 3, 128, None, torch.bfloat16),     # tiles before, across and after the queries
+    (1, 300, 1000, 3, 64, None, torch.float16),      # most keys after every query
+    (1, 1000, 130, 3, 128, None, torch.float16),     # most before; a tile of two keys
+    (60, 513, 511, 4, 128, (300, 140), torch.bfloat16),    # cut at both ends, several items per CTA
+    (60, 640, 640, 4, 64, (1, 400), torch.bfloat16),
+])
+def test_alibi_on_both_sides(cuda, B, Sq, Sk, H, D, window, dtype):
+    """Tiles on one side of their queries take another path than those in between, and slopes from
+    none to one that leaves a row little more than its own key. Reference in 64 bits: the scores carry
+    an fp32 rounding of their size, results and probabilities u of themselves."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(B, Sq, Sk, H, H, D, seed=Sq + Sk, dtype=dtype))
+    slopes = torch.tensor([0.0, 0.01, 0.3, 4.0], device=cuda)[-H:].contiguous()
+    out, lse = ops.attention(q, k, v, window=window, alibi_slopes=slopes, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    i, j = torch.arange(Sq, device=cuda)[:, None], torch.arange(Sk, device=cuda)[None]
+    u = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    for b in {0, B - 1}:
+        s = torch.einsum("ihd,jhd->hij", q[b].double(), k[b].double()) * D ** -0.5
+        s = s - slopes.double().view(-1, 1, 1) * (i - j).abs()
+        if window is not None:
+            s = s.masked_fill((j - i < -window[0]) | (j - i > window[1]), float("-inf"))
+        ref_lse = torch.logsumexp(s, -1)
+        seen = ~torch.isinf(ref_lse)
+        assert torch.equal(torch.isinf(lse[b]), ~seen)
+        # a score has up to 4 roundings of half an ulp of its terms; 1e-5 for dot products and sums
+        size = ref_lse.abs() + 10
+        assert bool(((lse[b].double() - ref_lse).abs()[seen] <= (1e-5 + 2.0 ** -22 * size)[seen]).all())
+        p = torch.softmax(s, -1).nan_to_num_(0.0)
+        ref = torch.einsum("hij,jhd->ihd", p, v[b].double())
+        bound = u * (ref.abs() + torch.einsum("hij,jhd->ihd", p, v[b].double().abs())) + 1e-4
+        assert bool(((out[b].double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("extra", [0, 1])  # one work item per SM, and one more
 @pytest.mark.parametrize("causal,alibi", [(False, False), (True, False), (False, True), (True, True)])
 @pytest.mark.parametrize("Sq,Sk,D", [(17, 1, 128), (130, 128, 64), (256, 129, 128), (200, 700, 128)])

@@ -51,17 +51,24 @@ constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
 constexpr unsigned AP_LAG = 1500;
 
 // What is added to the scaled scores: nothing; ALiBi as one ramp per row (every visible key at or
-// before its query); ALiBi on either side of the query, or a scale that is not positive.
-enum AttnBias { AP_NONE = 0, AP_RAMP = 1, AP_GENERAL = 2 };
+// before its query); ALiBi on either side of the query, or a scale that is not positive. Of the last,
+// a KV tile that lies on one side of its Q tile is a ramp as well, up or down, added to the raw score by
+// one packed FMA for two, counted from its key next to the queries (its last, AP_RAMP_TO_LAST, or its
+// first), so that the keys that weigh most carry the least rounding; only those in between take a difference, a product and an FMA for each score
+// (for all tiles: 4 x 2048, 32 / 8 heads x 128 382 us, so 323; 16 heads x 64 172, 148).
+enum AttnBias { AP_NONE = 0, AP_RAMP = 1, AP_GENERAL = 2, AP_RAMP_TO_LAST = 3 };
 
 // Registers per thread after the split. The four warpgroups' shares sum to what the launch gives
-// (4 x 128). The softmax loop holds 128 scores: with 168 it spills (16 x 4096 causal 2111 us against
-// 1947 with 176). Beyond that the register allocator's schedule decides, measured with 176 / 184:
-// plain scores at head dim 128: causal 1947 / 1874 us, window 1024 1189 / 1044, 2 x 8192 full 1953 /
-// 1731; with ALiBi 2153 / 2345; head dim 64, 8 x 2048 x 16 heads 226 / 239, causal 146 / 151.
-template <int D, int BIAS>
+// (4 x 128). The softmax loop holds 128 scores and does not fit 168 (16 x 4096 causal 2111 us against
+// 1947 with 176); with 176 and 184 a few values around the loop and in the epilogue are spilled.
+// Beyond that the register allocator's schedule decides, measured with 176 / 184: plain scores at head
+// dim 128: causal 1947 / 1874 us, window 1024 1189 / 1044, 2 x 8192 full 1953 / 1731; ALiBi on both
+// sides (ramps from column 0) 4 x 2048 339 / 313, but one item per CTA 51.3 / 55.5; ALiBi under a causal
+// mask 2153 / 2345; head dim 64, 8 x 2048 x 16 heads 226 / 239, causal 146 / 151.
+template <int D, int BIAS, bool SINGLE>
 struct PlainRegs {
-  static constexpr int SOFTMAX = D == 128 && BIAS == AP_NONE ? 184 : 176;
+  static constexpr bool WIDE = D == 128 && (BIAS == AP_NONE || (BIAS == AP_GENERAL && !SINGLE));
+  static constexpr int SOFTMAX = WIDE ? 184 : 176;
   static constexpr int EPILOGUE = 256 - SOFTMAX, OTHER = 256 - SOFTMAX;
   static_assert(2 * SOFTMAX + EPILOGUE + OTHER <= 512, "register split");
 };
@@ -71,15 +78,16 @@ struct PlainRegs {
 struct ColumnPairs {
   float2 v[ATT_BN / 2];
 };
-constexpr ColumnPairs column_pairs() {
+constexpr ColumnPairs column_pairs(int first) {
   ColumnPairs t{};
   for (int i = 0; i < ATT_BN / 2; ++i) {
-    t.v[i].x = static_cast<float>(2 * i);
-    t.v[i].y = static_cast<float>(2 * i + 1);
+    t.v[i].x = static_cast<float>(first + 2 * i);
+    t.v[i].y = static_cast<float>(first + 2 * i + 1);
   }
   return t;
 }
-static __constant__ ColumnPairs g_columns = column_pairs();
+static __constant__ ColumnPairs g_columns = column_pairs(0);
+static __constant__ ColumnPairs g_columns_to_last = column_pairs(1 - ATT_BN);
 
 template <int D>
 struct PlainSmem {
@@ -413,7 +421,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
   };
 
   if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::OTHER));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS, SINGLE>::OTHER));
     if (warp == 12) {
       // =========================== TMA producer =======================================
       if (lane == 0) {
@@ -601,7 +609,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     }
   } else if (warp >= 8) {
     // =========================== epilogue =============================================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::EPILOGUE));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS, SINGLE>::EPILOGUE));
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
     uint32_t opar[2] = {0u, 0u};  // parity of the next finished O
@@ -653,7 +661,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
     }
   } else {
     // =========================== softmax ==============================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS>::SOFTMAX));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PlainRegs<D, BIAS, SINGLE>::SOFTMAX));
     const int t = warp >> 2;
     const int wq = warp & 3;
     const int rl = wq * 32 + lane;
@@ -697,8 +705,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         lo_i = max(0, row - p.win_left);
         lo_max = max(0, row1 - p.win_left);
       }
-      const float unit = BIAS == AP_GENERAL ? 1.0f : sl2;
-      const float kc = BIAS == AP_RAMP ? __fdividef(slope2, sl2) : 0.0f;
+      const float kc = BIAS == AP_NONE ? 0.0f : __fdividef(slope2, sl2);
+      // whether scores can carry the ramp: scaled by a positive number, and not too small a one
+      const bool foldable = BIAS == AP_GENERAL && sl2 > 0.0f && fabsf(kc) < 1e30f;
       // The row sum in four shares, one of every fourth pair of columns; in a tile each is a chain of
       // the 16 even and one of the 16 odd columns. The order of attention.cu, whose rows are held by
       // four threads, so that the two agree to the last bit. Two chains and one share, 2 to 3 us in 200
@@ -723,23 +732,29 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         tc_fence_after();
         // by a vote: a branch that the compiler knows to be uniform
         const bool cut = __any_sync(0xffffffffu, c0 + BN - 1 > hi_min || c0 < lo_max);
+        // AP_GENERAL: a tile that lies on one side of its queries is a ramp too
+        const bool up = BIAS == AP_GENERAL && __any_sync(0xffffffffu, foldable && c0 + BN - 1 <= row0);
+        const bool down = BIAS == AP_GENERAL && __any_sync(0xffffffffu, foldable && c0 >= row1);
+        const float unit = BIAS == AP_GENERAL && !up && !down ? 1.0f : sl2;
         uint32_t sr[BN];
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
         // 32 columns: add the bias, hide what the row does not see, take the maximum
-        auto take = [&](auto off_tag, auto cut_tag) {
-          constexpr int OFF = decltype(off_tag)::value;
-          if constexpr (BIAS == AP_GENERAL) {
+        auto take = [&](auto off_tag, auto cut_tag, auto bias_tag) {
+          constexpr int OFF = decltype(off_tag)::value, TILE_BIAS = decltype(bias_tag)::value;
+          if constexpr (TILE_BIAS == AP_GENERAL) {
             const float fi = static_cast<float>(row - c0);
 #pragma unroll
             for (int c = OFF; c < OFF + 32; ++c)
               sr[c] = __float_as_uint(fmaf(-slope2, fabsf(fi - static_cast<float>(c)),
                                            __uint_as_float(sr[c]) * sl2));
           }
-          if constexpr (BIAS == AP_RAMP) {
-            const float2 kc2 = make_float2(kc, kc);
+          if constexpr (TILE_BIAS == AP_RAMP || TILE_BIAS == AP_RAMP_TO_LAST) {
+            const float kt = BIAS == AP_GENERAL && TILE_BIAS == AP_RAMP ? -kc : kc;
+            const float2 kc2 = make_float2(kt, kt);
 #pragma unroll
             for (int c = OFF; c < OFF + 32; c += 2)
-              put_pair(sr + c, fma2(g_columns.v[c / 2], kc2, pair_of(sr + c)));
+              put_pair(sr + c, fma2(TILE_BIAS == AP_RAMP ? g_columns.v[c / 2] : g_columns_to_last.v[c / 2],
+                                    kc2, pair_of(sr + c)));
           }
           if constexpr (decltype(cut_tag)::value) {
             const int hi_c = hi_i - c0 - OFF, lo_c = lo_i - c0 - OFF;
@@ -757,23 +772,31 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             for (int i = 0; i < 4; ++i)
               mx[i] = max3(mx[i], __uint_as_float(sr[c + 2 * i]), __uint_as_float(sr[c + 2 * i + 1]));
         };
-        auto take_all = [&](auto cut_tag) {
+        auto take_all = [&](auto cut_tag, auto bias_tag) {
           tmem_wait_ld32<0>(sr);
           tmem_ld32<32>(s_addr + 32, sr);
-          take(std::integral_constant<int, 0>{}, cut_tag);
+          take(std::integral_constant<int, 0>{}, cut_tag, bias_tag);
           tmem_wait_ld32<32>(sr);
           tmem_ld32<64>(s_addr + 64, sr);
-          take(std::integral_constant<int, 32>{}, cut_tag);
+          take(std::integral_constant<int, 32>{}, cut_tag, bias_tag);
           tmem_wait_ld32<64>(sr);
           tmem_ld32<96>(s_addr + 96, sr);
-          take(std::integral_constant<int, 64>{}, cut_tag);
+          take(std::integral_constant<int, 64>{}, cut_tag, bias_tag);
           tmem_wait_ld32<96>(sr);
-          take(std::integral_constant<int, 96>{}, cut_tag);
+          take(std::integral_constant<int, 96>{}, cut_tag, bias_tag);
         };
         tmem_ld32<0>(s_addr, sr);
-        if (cut) take_all(std::true_type{});
-        else take_all(std::false_type{});
-        const float off = BIAS == AP_RAMP ? slope2 * static_cast<float>(c0 - row) : 0.0f;
+        auto take_tile = [&](auto bias_tag) {
+          if (cut) take_all(std::true_type{}, bias_tag);
+          else take_all(std::false_type{}, bias_tag);
+        };
+        if (BIAS == AP_GENERAL && up) take_tile(std::integral_constant<int, AP_RAMP_TO_LAST>{});
+        else if (BIAS == AP_GENERAL && down) take_tile(std::integral_constant<int, AP_RAMP>{});
+        else take_tile(std::integral_constant<int, BIAS>{});
+        // the bias of the tile's column 0 (AP_RAMP_TO_LAST: of its last): slope_v * dist
+        const float slope_v = BIAS == AP_GENERAL ? (up ? slope2 : down ? -slope2 : 0.0f) : slope2;
+        const float dist = static_cast<float>((up ? c0 + BN - 1 : c0) - row);
+        const float off = BIAS == AP_NONE ? 0.0f : slope_v * dist;
         const float m_raw = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
         const float m_tile = fmaf(m_raw, unit, off);  // unit > 0: -inf stays -inf
 
@@ -799,7 +822,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             }
           }
         }
-        const float neg = off - m_ref;
+        const float neg = BIAS == AP_GENERAL ? fmaf(slope_v, dist, -m_ref) : off - m_ref;
 
         // P = exp2(x - m), 32 keys (16 packed columns) at a time, over the scores
         static_assert(AP_REST == 2, "the last 32 keys are two MMAs");
@@ -883,7 +906,7 @@ static int launch_plain(const AttnParams& p, cudaStream_t stream) {
     if (cudaFuncGetAttributes(&a, attn_plain_kernel<D, BF16, BIAS, SINGLE>) != cudaSuccess)
       return TRX_ERR_CUDA;
     // the register split draws on what the block is launched with: never wait for more than that
-    using Regs = PlainRegs<D, BIAS>;
+    using Regs = PlainRegs<D, BIAS, SINGLE>;
     if (a.numRegs * 4 < 2 * Regs::SOFTMAX + Regs::EPILOGUE + Regs::OTHER) return TRX_ERR_UNSUPPORTED;
     if (cudaFuncSetAttribute(attn_plain_kernel<D, BF16, BIAS, SINGLE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
