@@ -48,14 +48,18 @@ constexpr int AP_REST = 2;  // of the 8 MMAs of a P V, those of the second piece
 // 256 on 1024 15.6, 15.2). 1000 / 1250 / 1750 cycles: 109.3 / 108.5 / 108.7, 1 x 1000 25.4 / 22.9 /
 // 21.8, 2 x 256 11.5 / 11.2 / 11.2. The same in launches of several items per CTA gained 1 to 3 % on
 // some and lost as much on others. A single visit (up to 128 keys) has nobody to get out of step with.
-constexpr unsigned AP_LAG = 1500;
+// A bias makes the softmax, and so half a visit, longer: 1500 / 1900 / 2200 / 2600 cycles, causal with
+// ALiBi 1 x 1000 26.5 / 25.1 / 24.5 / 24.6, 4 x 512 18.7 / 17.4 / 17.1 / 17.2, both sides 1 x 2048,
+// 8 heads 51.3 / 50.0 / 49.3 / 50.3.
+constexpr unsigned AP_LAG = 1500, AP_LAG_BIAS = 2200;
 
 // What is added to the scaled scores: nothing; ALiBi as one ramp per row (every visible key at or
 // before its query); ALiBi on either side of the query, or a scale that is not positive. Of the last,
 // a KV tile that lies on one side of its Q tile is a ramp as well, up or down, added to the raw score by
 // one packed FMA for two, counted from its key next to the queries (its last, AP_RAMP_TO_LAST, or its
-// first), so that the keys that weigh most carry the least rounding; only those in between take a difference, a product and an FMA for each score
-// (for all tiles: 4 x 2048, 32 / 8 heads x 128 382 us, so 323; 16 heads x 64 172, 148).
+// first), so that the keys that weigh most carry the least rounding; only those in between take a
+// difference, a product and an FMA for each score (for all tiles: 4 x 2048, 32 / 8 heads x 128 382 us,
+// so 323; 16 heads x 64 172, 148).
 enum AttnBias { AP_NONE = 0, AP_RAMP = 1, AP_GENERAL = 2, AP_RAMP_TO_LAST = 3 };
 
 // Registers per thread after the split. The four warpgroups' shares sum to what the launch gives
@@ -724,8 +728,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
         s_par ^= 1u;
         if (SINGLE && t == 1 && itn == 0 && n_it > 1) {
           // half a visit behind the other Q tile, see AP_LAG
+          constexpr unsigned LAG = BIAS == AP_NONE ? AP_LAG : AP_LAG_BIAS;
           const unsigned begin = static_cast<unsigned>(clock());
-          for (int i = 0; i < 4096 && static_cast<unsigned>(clock()) - begin < AP_LAG; ++i) {
+          for (int i = 0; i < 4096 && static_cast<unsigned>(clock()) - begin < LAG; ++i) {
           }
           __syncwarp();
         }
