@@ -537,6 +537,32 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("B,S,Hq,Hk", [
+    (4, 2500, 32, 8),    # 41 MB of keys and values, 10 of a batch: all heads of a batch at a time
+    (1, 6151, 32, 32),   # 101 MB of a batch: one head after the other, row pairs, heaviest first
+])
+def test_causal_orders_of_large_calls(cuda, B, S, Hq, Hk):
+    """Causal calls whose keys and values do not fit L2 walk their work items in other orders. Rows at
+    the edges of the tiles and some in between, against fp32 on the device."""
+    from trinix_b200 import ops
+    D = 128
+    q, k, v = (t.to(cuda) for t in _qkv(B, S, S, Hq, Hk, D, seed=S))
+    out, lse = ops.attention(q, k, v, causal=True, return_lse=True)
+    assert T.attention_status(cuda) == 0
+    rows = torch.tensor(sorted({r for e in range(0, S + 1, 128) for r in (e - 1, e, e + 77)
+                                if 0 <= r < S} | {S - 1}), device=cuda)
+    hidden = torch.arange(S, device=cuda)[None] > rows[:, None]
+    for b in range(B):
+        for h in range(Hq):
+            kf, vf = k[b, :, h * Hk // Hq].float(), v[b, :, h * Hk // Hq].float()
+            s = (q[b, rows, h].float() @ kf.t() * D ** -0.5).masked_fill(hidden, float("-inf"))
+            p = torch.softmax(s, -1)
+            ref, size = p @ vf, p @ vf.abs()
+            assert bool(((out[b, rows, h].float() - ref).abs()
+                         <= 2.0 ** -8 * (ref.abs() + size) + 1e-4).all()), (b, h)
+            assert float((lse[b, h, rows] - torch.logsumexp(s, -1)).abs().max()) <= 1e-4, (b, h)
+
+
 @pytest.mark.parametrize("B,Sq,Sk,H,D,window,dtype", [
     (1, 256, 256, 3, 128, None, torch.bfloat16),     # tiles before, across and after the queries
     (1, 300, 1000, 3, 64, None, torch.float16),      # most keys after every query

@@ -947,8 +947,11 @@ int launch_attn_plain(AttnParams& p, int64_t D, cudaStream_t stream) {
   const bool single = m * h * p.B <= sm_count_of_current_device();
   p.order = AP_MHB;
   if (p.causal && m <= 65535) {
-    // Heaviest row blocks first (one head after the other, 2 x 4096 x 32 / 8 heads: 283 us, so 255),
-    // over all heads whose keys and values fit a third of L2, or those of one batch.
+    // Heaviest row blocks first: over all heads of all batches while their keys and values are a third
+    // of L2, over those of one batch up to 100 MB. One head after the other / one batch / all, us:
+    // 4 x 2048, 32 / 8 heads x 128 (34 MB) 158 / 147 / 144, 2 x 4096 (34 MB) 269 / 248 / 248, 8 x 2048
+    // (67 MB) 292 / 286 / 288, 16 x 4096 (268 MB, 17 of a batch) 2174 / 2166 / 2374. The upper line is
+    // not fitted: 1 x 8192, 32 / 32 heads (134 MB) takes 546 / 490 / 489, 1 x 6144 (101 MB) 334 / 286 / 285.
     const double kv = 4.0 * p.Sk * static_cast<double>(D) * p.Hq / p.group;  // bytes of a batch
     if (kv * p.B <= 40e6) p.order = AP_HBM;
     else if (kv <= 100e6) p.order = AP_HMB;
