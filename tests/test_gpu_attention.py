@@ -537,6 +537,58 @@ def test_few_query_rows_with_every_number_of_splits(cuda, B, Sq, Sk, Hq, Hk, D):
     assert float((lse - ref_lse).abs().max()) <= 5e-5 + Sk * 2.0 ** -24
 
 
+@pytest.mark.parametrize("causal,window,alibi,scale", [
+    (False, None, False, None), (True, None, False, None), (False, (5, 9), False, None),
+    (False, (200, 0), True, None), (True, None, True, None), (False, None, True, None),
+    (False, None, False, -0.1), (True, None, True, -0.1), (False, None, False, 0.0),
+])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hk,D,dtype", [
+    (2, 128, 128, 8, 2, 128, torch.bfloat16), (3, 300, 127, 4, 4, 64, torch.float16),
+    (1, 33, 1, 6, 3, 128, torch.float16), (1, 16, 97, 32, 8, 128, torch.bfloat16),
+    (2, 257, 65, 4, 4, 128, torch.bfloat16),
+])
+def test_single_key_tile(cuda, B, Sq, Sk, Hq, Hk, D, dtype, causal, window, alibi, scale):
+    """Calls of one KV tile have a kernel of their own up to a wave of CTAs: every form that they take,
+    contiguous, in other layouts and as part of a batch of more than a wave (bit for bit the same).
+    Reference in 64 bits, bounds as in test_alibi_on_both_sides."""
+    from trinix_b200 import ops
+    q, k, v = (t.to(cuda) for t in _qkv(B, Sq, Sk, Hq, Hk, D, seed=Sq + Sk, dtype=dtype))
+    slopes = R.alibi_slopes_ref(Hq).to(cuda) if alibi else None
+    kw = dict(causal=causal, window=window, alibi_slopes=slopes, scale=scale, return_lse=True)
+    out, lse = ops.attention(q, k, v, **kw)
+    swap = lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)  # noqa: E731
+    cache = torch.full((B, 200, Hk, D), float("nan"), device=cuda, dtype=dtype)
+    cache[:, 40:40 + Sk] = v  # the values around the slice are never used
+    again = ops.attention(swap(q), swap(k), cache[:, 40:40 + Sk], **kw)
+    assert T.attention_status(cuda) == 0
+    assert torch.equal(again[0], out) and torch.equal(again[1], lse)
+    if Sq > 16:  # the number of key splits of fewer rows goes by the batch
+        n = torch.cuda.get_device_properties(cuda).multi_processor_count
+        more = ops.attention(q.repeat(n, 1, 1, 1), k.repeat(n, 1, 1, 1), v.repeat(n, 1, 1, 1), **kw)
+        assert torch.equal(more[0][:B], out) and torch.equal(more[1][-B:], lse)
+    g = Hq // Hk
+    s = torch.einsum("bihd,bjhd->bhij", q.double(), k.double().repeat_interleave(g, 2))
+    s = s * (D ** -0.5 if scale is None else scale)
+    i, j = torch.arange(Sq, device=cuda)[:, None], torch.arange(Sk, device=cuda)[None]
+    if alibi:
+        s = s - slopes.double().view(1, -1, 1, 1) * (i - j).abs()
+    if causal:
+        s = s.masked_fill(j > i, float("-inf"))
+    if window is not None:
+        s = s.masked_fill((j - i < -window[0]) | (j - i > window[1]), float("-inf"))
+    ref_lse = torch.logsumexp(s, -1)
+    seen = ~torch.isinf(ref_lse)
+    assert torch.equal(torch.isinf(lse), ~seen)
+    assert bool(((lse.double() - ref_lse).abs()[seen]
+                 <= (1e-5 + 2.0 ** -22 * (ref_lse.abs() + 10))[seen]).all())
+    p, vt = torch.softmax(s, -1).nan_to_num_(0.0), v.double().repeat_interleave(g, 2)
+    ref = torch.einsum("bhij,bjhd->bihd", p, vt)
+    u = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    bound = u * (ref.abs() + torch.einsum("bhij,bjhd->bihd", p, vt.abs())) + 1e-4
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    assert not out[~seen.transpose(1, 2)].any()
+
+
 @pytest.mark.parametrize("B,S,Hq,Hk", [
     (4, 2500, 32, 8),    # 41 MB of keys and values, 10 of a batch: all heads of a batch at a time
     (1, 6151, 32, 32),   # 101 MB of a batch: one head after the other, row pairs, heaviest first

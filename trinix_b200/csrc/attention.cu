@@ -31,8 +31,9 @@
 
 namespace trx {
 
-// What an instantiation carries: dropout; a dense additive mask with or without dropout.
-enum AttnFeature { ATT_DROPOUT = 1, ATT_MASK_F32 = 2, ATT_MASK_16 = 3 };
+// What an instantiation carries: neither (calls of a single KV tile, see is_short); dropout; a dense
+// additive mask with or without dropout.
+enum AttnFeature { ATT_SHORT = 0, ATT_DROPOUT = 1, ATT_MASK_F32 = 2, ATT_MASK_16 = 3 };
 __host__ __device__ constexpr bool feature_has_mask(int f) { return f >= ATT_MASK_F32; }
 
 // With a mask each softmax warp has MASK_BUFS buffers of 16 rows x 32 mask values; at head dim 128
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
 
       const bool need_mask = (c0 + ATT_BN - 1 > hi_min) || (c0 < lo_max);
       float m_tile[2] = {-INFINITY, -INFINITY};
+      float dist[2] = {0.0f, 0.0f};  // ATT_SHORT: x = t * sl2 + slope2 * dist
       auto max_of_tile = [&] {
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
@@ -479,9 +481,50 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
                        __uint_as_float(sr[4 * g + 5 + 2 * hr]));
           }
           m_tile[hr] = fmaxf(mx0, mx1);
+          if (FEATURE == ATT_SHORT) m_tile[hr] = fmaf(m_tile[hr], sl2, slope2 * dist[hr]);  // sl2 > 0
         }
       };
-      {
+      if constexpr (FEATURE == ATT_SHORT) {
+        // Scores stay raw. Every visible key is at or before its query: ALiBi is a ramp over the columns
+        // that folds into them and a constant of the row. The arithmetic is attention_plain.cu's, operation
+        // by operation, so that a call's bits do not go by the size of its batch. What the compiler spills
+        // decides: 8 bytes this way; 70 to 100 with the columns as a running pair, or without ALiBi in this
+        // instantiation (2 x 64 x 64, 32 / 8 heads x 128 8.3 us, 8.8, 8.9).
+        if (need_mask) {
+          const bool cut_lo = c0 < lo_max;  // one comparison per score where only the upper end is cut
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {
+            const int lo_c = lo_i[hr] - c0 - 2 * q4, hi_c = hi_i[hr] - c0 - 2 * q4;
+            auto hide = [&](auto hidden) {
+#pragma unroll
+              for (int g = 0; g < 16; ++g)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                  if (hidden(8 * g + e)) sr[4 * g + 2 * hr + e] = 0xff800000u;
+            };
+            if (cut_lo) hide([&](int c) { return c < lo_c || c > hi_c; });
+            else hide([&](int c) { return c > hi_c; });
+          }
+        }
+        if (has_alibi) {
+          const float kc = __fdividef(slope2, sl2);
+          const float2 kc2 = make_float2(kc, kc);
+          const float2 column = make_float2(static_cast<float>(2 * q4), static_cast<float>(2 * q4 + 1));
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {
+            dist[hr] = static_cast<float>(c0 - row_g[hr]);
+#pragma unroll
+            for (int g = 0; g < 16; ++g) {
+              const int i = 4 * g + 2 * hr;
+              const float2 t = fma2(add2(column, make_float2(8.0f * g, 8.0f * g)), kc2,
+                                    make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])));
+              sr[i] = __float_as_uint(t.x);
+              sr[i + 1] = __float_as_uint(t.y);
+            }
+          }
+        }
+        max_of_tile();
+      } else {
         // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf. Dropout without a
         // mask does the same, every path fixed at compile time: 2 x 4096^2, 16 / 4 heads, head dim
         // 128, 858 us (causal 523). Left to run-time flags beside the plain paths its 96 registers
@@ -610,15 +653,17 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
           }
         }
       } else {
-        const float2 nm2[2] = {make_float2(-m_ref[0], -m_ref[0]),
-                               make_float2(-m_ref[1], -m_ref[1])};
+        const float nm[2] = {FEATURE == ATT_SHORT ? fmaf(slope2, dist[0], -m_ref[0]) : -m_ref[0],
+                             FEATURE == ATT_SHORT ? fmaf(slope2, dist[1], -m_ref[1]) : -m_ref[1]};
+        const float2 nm2[2] = {make_float2(nm[0], nm[0]), make_float2(nm[1], nm[1])};
 #pragma unroll
         for (int g = 0; g < 16; ++g) {
 #pragma unroll
           for (int hr = 0; hr < 2; ++hr) {
-            const float2 x = add2(make_float2(__uint_as_float(sr[4 * g + 2 * hr]),
-                                              __uint_as_float(sr[4 * g + 2 * hr + 1])),
-                                  nm2[hr]);
+            const float2 s2 = make_float2(__uint_as_float(sr[4 * g + 2 * hr]),
+                                          __uint_as_float(sr[4 * g + 2 * hr + 1]));
+            const float2 x = FEATURE == ATT_SHORT ? fma2(s2, make_float2(sl2, sl2), nm2[hr])
+                                                  : add2(s2, nm2[hr]);
             const float2 pe = make_float2(fast_exp2(x.x), fast_exp2(x.y));
             lsum[hr] = add2(lsum[hr], pe);
             sr[2 * g + hr] = pack16<BF16>(pe.x, pe.y);
@@ -833,7 +878,23 @@ template <int D, bool BF16>
 static int launch_attn(const AttnParams& p, cudaStream_t stream) {
   if (p.bias_kind == 1) return launch_attn_feature<D, BF16, ATT_MASK_F32>(p, stream);
   if (p.bias_kind == 2) return launch_attn_feature<D, BF16, ATT_MASK_16>(p, stream);
-  return launch_attn_feature<D, BF16, ATT_DROPOUT>(p, stream);
+  if (p.drop_thr) return launch_attn_feature<D, BF16, ATT_DROPOUT>(p, stream);
+  return launch_attn_feature<D, BF16, ATT_SHORT>(p, stream);
+}
+
+// Calls without mask or dropout that take this kernel and not attention_plain.cu's: one KV tile, and no
+// more CTAs than SMs. A single visit has no other to overlap with, and 16 softmax warps with half a row
+// per thread are through it sooner than 8 with a row. This / the other kernel, us, head dim 128, 32 / 8
+// heads: 1 x 17 queries x 128 keys 7.3 / 8.2, causal 7.7 / 8.8, with ALiBi 8.1 / 9.5; 2 x 64 x 64 8.3 /
+// 8.7, causal 8.6 / 9.0; 4 x 128 x 128, 16 / 2 heads 9.9 / 9.9, causal with ALiBi 10.6 / 11.2; 1 x 1024 x
+// 128 10.0 / 10.2; 1 x 256 x 128 causal, 16 heads (row pairs) 10.2 / 9.6; head dim 64, 16 heads 8 x 128 x
+// 128 6.8 / 7.1. ALiBi on both sides (4 x 128 x 128 11.0 / 11.0 when this kernel took it) and scales that
+// are not positive need another form of the scores and stay there.
+static bool is_short(const AttnParams& p) {
+  const int64_t rows = p.pair_heads ? ATT_BM : ATT_NQ * ATT_BM, heads = p.pair_heads ? p.Hq / 2 : p.Hq;
+  return p.Sk > 0 && p.Sk <= ATT_BN && p.scale_log2 > 0.0f &&
+         (!p.slopes || p.causal || p.win_right == 0) &&
+         (p.Sq + rows - 1) / rows * heads * p.B <= sm_count_of_current_device();
 }
 
 }  // namespace trx
@@ -986,7 +1047,7 @@ static int attn_fwd_launch(AttnParams& p, int64_t D, void* stream) {
     return p.is_bf16 ? (wide ? launch_decode<64, true, 2>(p, s) : launch_decode<64, true, 1>(p, s))
                      : (wide ? launch_decode<64, false, 2>(p, s) : launch_decode<64, false, 1>(p, s));
   }
-  if (p.plain) return launch_attn_plain(p, D, s);
+  if (p.plain && !is_short(p)) return launch_attn_plain(p, D, s);
   if (D == 128) return p.is_bf16 ? launch_attn<128, true>(p, s) : launch_attn<128, false>(p, s);
   return p.is_bf16 ? launch_attn<64, true>(p, s) : launch_attn<64, false>(p, s);
 }

@@ -469,13 +469,14 @@ static int launch_decode(const AttnParams& p, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? TRX_OK : TRX_ERR_CUDA;
 }
 
-// Calls that take this kernel: up to 16 query rows. The tcgen05 kernel spends the same time on any
-// Sq up to 128 (it works on whole 128-row tiles), this one works on tiles of 16 packed rows.
-// Measured at 4096 keys, head dim 128, this / the tcgen05 kernel: Sq = 16, B = 16, 32 / 32 heads
-// 159 / 269 us; 32 / 8 heads 91 / 140 us; 32 / 1 heads (512 packed rows) 88 / 139 us, B = 1 29 / 69
-// us; Sq = 64, B = 4, 32 / 8 heads 90 / 71 us. The exception is a single key tile of the tcgen05 kernel
-// that is nearly full, in one wave of CTAs, at head dim 128, against two row tiles per warp here: 97
-// to 128 keys 8.4 to 8.8 / 7.6 to 8.2 us whatever the batch (96 keys 8.3 / 8.2; 129 keys 9.1 / 10.6).
+// Calls that take this kernel: up to 16 query rows. The tcgen05 kernels spend the same time on any
+// Sq up to 128 (they work on whole 128-row tiles), this one works on tiles of 16 packed rows. Measured
+// at 4096 keys, head dim 128, this / attention_plain.cu: Sq = 16, B = 16, 32 / 32 heads 160 / 198 us;
+// 32 / 8 heads 94 / 139 us; 32 / 1 heads (512 packed rows) 90 / 138 us, B = 1 29 / 56 us; Sq = 32, B = 4,
+// 32 / 8 heads 52 / 57, Sq = 64 89 / 57 us. The exception is a single key tile of attention.cu's kernel
+// that is nearly full, in one wave of CTAs, at head dim 128, against two row tiles per warp here: 97 to
+// 128 keys 8.4 to 8.7 / 7.3 to 7.8 us (96 keys 8.1 to 8.4 / 7.6 to 7.9, 64 keys 7.3 / 7.4; 129 keys 9.2 /
+// 10.0).
 static bool use_decode(const AttnParams& p, int64_t D) {
   const int64_t rows = static_cast<int64_t>(p.Sq) * p.group;
   if (p.Sq > 16 || (p.Hq / p.group) * ((rows + 15) / 16) > 65535) return false;

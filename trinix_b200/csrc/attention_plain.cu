@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             }
           }
         }
-        const float neg = BIAS == AP_GENERAL ? fmaf(slope_v, dist, -m_ref) : off - m_ref;
+        const float neg = BIAS == AP_NONE ? off - m_ref : fmaf(slope_v, dist, -m_ref);
 
         // P = exp2(x - m), 32 keys (16 packed columns) at a time, over the scores
         static_assert(AP_REST == 2, "the last 32 keys are two MMAs");
