@@ -1,6 +1,7 @@
-// Attention forward with a dense additive mask or dropout, and the host side of every attention call:
-// softmax(scale * Q K^T + bias) V with online softmax. Calls without either run attention_plain.cu or,
-// with up to 16 query rows, attention_decode.cuh (but for a few, see use_decode).
+// Attention forward with a dense additive mask or dropout, or of a single KV tile, and the host side of
+// every attention call: softmax(scale * Q K^T + bias) V with online softmax. Other calls without mask or
+// dropout run attention_plain.cu or, with up to 16 query rows, attention_decode.cuh (but for a few, see
+// use_decode).
 //
 // One CTA owns two 128-row Q tiles that ping-pong on the tensor pipe: the same 128 query rows of
 // two query heads that share a kv head (GQA / MQA: both tiles then see exactly the same keys), or
@@ -15,14 +16,15 @@
 //               and O += P V (P read from TMEM, V from shared memory, MN-major); one thread,
 //               flat scalar code, specialised for the rounds in which both Q tiles are active
 // TMEM (512 columns): S0 | S1 | O0 | O1, 128 fp32 columns each; P (16-bit) overwrites the
-// first 64 columns of its S. The softmax groups read S with tcgen05.ld, exponentiate with
-// exp2 (scale*log2e folded into one FMA, ALiBi as one more), write P back with tcgen05.st,
-// rescale O in TMEM only when the running row max grew by more than 2^8 (lazy rescale) and
-// run the epilogue (O / l -> global). KV tiles outside the causal / window range of a Q tile
-// are never visited; masks are applied only on boundary tiles. Query head h reads kv head
+// first 64 columns of its S. The softmax groups read S with tcgen05.ld, form the scores in the
+// log2 domain in place (scaled, ALiBi and mask added; of a single KV tile they stay raw and are
+// scaled in the exponent's FMA), write P = exp2(x - max) back with tcgen05.st, rescale O in TMEM
+// only when the running row max grew by more than 2^8 (lazy rescale) and run the epilogue
+// (O / l -> global). KV tiles outside the causal / window range of a Q tile are never visited;
+// causal and window limits are applied only on boundary tiles. Query head h reads kv head
 // h / (Hq / Hk), so GQA / MQA need no tiled copies. With ALiBi under a causal mask the KV tiles
 // of a row block are visited from the diagonal backwards: the bias grows with the key index, so
-// in that order the first tile holds the row maximum and O is never rescaled again.
+// in that order (but for what a mask adds) the first tile holds the row maximum.
 //
 // Every wait on an mbarrier is bounded: after a fixed number of polls the kernel records a
 // code in the status word of the caller's workspace, raises a CTA-wide abort flag, drains its
@@ -30,6 +32,10 @@
 #include "attention_common.cuh"
 
 namespace trx {
+
+constexpr int ATT_STAGES = 4;     // KV ring depth (K and V tiles alternate)
+constexpr int ATT_SM_WARPS = 16;    // softmax warps: two warpgroups per Q tile, half a row per thread
+constexpr int ATT_THREADS = (ATT_SM_WARPS + 2) * 32;
 
 // What an instantiation carries: neither (calls of a single KV tile, see is_short); dropout; a dense
 // additive mask with or without dropout.
@@ -527,7 +533,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
       } else {
         // x = scale * log2e * s (ALiBi) + log2e * mask, in place; -inf stays -inf. Dropout without a
         // mask does the same, every path fixed at compile time: 2 x 4096^2, 16 / 4 heads, head dim
-        // 128, 858 us (causal 523). Left to run-time flags beside the plain paths its 96 registers
+        // 128, 858 us (causal 523). Left to run-time flags beside paths without either its 96 registers
         // spill in the generator's loop: 1470 us (887); one instantiation for masks and dropout with
         // a flag for each: 1097 us (673).
         const float2 scale2 = make_float2(sl2, sl2);

@@ -14,9 +14,6 @@ namespace trx {
 constexpr int ATT_BM = 128;       // rows per Q tile
 constexpr int ATT_BN = 128;       // keys per KV tile
 constexpr int ATT_NQ = 2;         // Q tiles per CTA
-constexpr int ATT_STAGES = 4;     // KV ring depth (K and V tiles alternate)
-constexpr int ATT_SM_WARPS = 16;    // softmax warps: two warpgroups per Q tile, half a row per thread
-constexpr int ATT_THREADS = (ATT_SM_WARPS + 2) * 32;
 constexpr uint32_t ATT_WAIT_LIMIT = 1u << 26;  // hard cap on polls per wait
 constexpr uint64_t ATT_WAIT_NS = 400ull * 1000 * 1000;  // wall-time budget of one wait
 constexpr float ATT_LAZY_RESCALE = 8.0f;       // log2 units
@@ -112,18 +109,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Without the suspension of try_wait: whether the phase is complete now.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -148,91 +133,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   atomicOr(status, code);
   return false;
-}
-// The same for a whole converged warp, whose lanes all poll: every branch here goes by a vote, so that
-// the compiler knows that the warp stays together and keeps what follows in uniform registers.
-__device__ __forceinline__ bool mbar_poll_warp(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag, unsigned int* status,
-                                               unsigned code) {
-  uint64_t t0 = 0;
-#pragma unroll 1
-  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    if ((i & 63u) == 63u) {
-      if (t0 == 0) t0 = global_ns();
-      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-      if (__any_sync(0xffffffffu, global_ns() - t0 > ATT_WAIT_NS)) break;
-    }
-  }
-  *abort_flag = 1;
-  atomicOr(status, code);
-  return false;
-}
-static __device__ __noinline__ bool mbar_poll_warp_call(uint32_t bar, uint32_t parity,
-                                                        volatile int* abort_flag,
-                                                        unsigned int* status, unsigned code) {
-  return mbar_poll_warp(bar, parity, abort_flag, status, code);
-}
-// `INLINE` false: out of line but for the first poll (which the hardware suspends for a while), for
-// roles with few live registers: the code of a role that has to react fast stays small.
-template <bool INLINE>
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag, unsigned int* status,
-                                               unsigned code) {
-  if constexpr (INLINE) return mbar_poll_warp(bar, parity, abort_flag, status, code);
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return __any_sync(0xffffffffu, mbar_poll_warp_call(bar, parity, abort_flag, status, code));
-}
-// A wait for something that takes as long as a whole work item (its row statistics, the next item): an
-// item may have any number of KV tiles, so the time counts from the last `progress` of the CTA.
-__device__ __forceinline__ bool mbar_poll_item(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag, unsigned int* status,
-                                               unsigned code, volatile int* progress) {
-  uint64_t t0 = 0;
-  int seen = 0;
-#pragma unroll 1
-  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    if ((i & 63u) == 63u) {
-      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-      const int now = *progress;
-      if (__any_sync(0xffffffffu, t0 == 0 || now != seen)) {
-        seen = now;
-        t0 = global_ns();
-        i = 0;
-      } else if (__any_sync(0xffffffffu, global_ns() - t0 > ATT_WAIT_NS)) {
-        break;
-      }
-    }
-  }
-  *abort_flag = 1;
-  atomicOr(status, code);
-  return false;
-}
-static __device__ __noinline__ bool mbar_poll_item_call(uint32_t bar, uint32_t parity,
-                                                        volatile int* abort_flag,
-                                                        unsigned int* status, unsigned code,
-                                                        volatile int* progress) {
-  return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
-}
-template <bool INLINE>
-__device__ __forceinline__ bool mbar_wait_item(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag, unsigned int* status,
-                                               unsigned code, volatile int* progress) {
-  if constexpr (INLINE) return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return __any_sync(0xffffffffu,
-                    mbar_poll_item_call(bar, parity, abort_flag, status, code, progress));
-}
-// One lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t is;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(is));
-  return is != 0;
 }
 // The status word's copy in host memory, if trx_attn_mirror attached one (workspace words 1 to 3:
 // a tag and the address). Written only by a launch that gave up or found a recorded failure, so a

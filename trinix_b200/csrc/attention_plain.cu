@@ -1,10 +1,12 @@
-// Attention forward without a dense mask or dropout: softmax(scale * Q K^T - ALiBi) V, online softmax.
+// Attention forward without a dense mask or dropout: softmax(scale * Q K^T - ALiBi) V, online softmax
+// (but few query rows: attention_decode.cuh, and a single KV tile in one wave of CTAs: attention.cu).
 //
 // A work item is two 128-row Q tiles: the same 128 query rows of two query heads that share a kv head
 // (GQA / MQA: both tiles then see exactly the same keys), or 256 consecutive rows of one head
 // otherwise. A CTA (one per SM) works on the item of its own block index and then on further ones
 // that the hardware hands it (cluster launch control), so that set-up is paid once per SM and the next
-// item's copies, first Q K^T and softmax run under the epilogue of the last. 16 warps:
+// item's copies, first Q K^T and softmax run under the epilogue of the last; launches of one item per CTA
+// have instantiations of their own. 16 warps:
 //   warps 0-3, 4-7  softmax of Q tile 0 and 1, a thread per row (TMEM lane): no shuffles
 //   warps 8-11      epilogue: O / l -> global
 //   warp 12         TMA producer: Q, then K and V tiles of 128 keys through a 4-stage ring, across
@@ -20,18 +22,20 @@
 //
 // What bounds it: per Q tile a chain scores -> softmax (about 2000 cycles, of them 1024 on the
 // special-function unit) -> P V -> next Q K^T (1032 cycles at the MMA rate) -> scores; two of them
-// share the SM, the tensor and the special-function pipe are each busy 55 to 60 % of the time, under
-// the power cap. What mattered (16 x 4096 causal, 32 / 8 heads x 128 unless said otherwise):
+// share the SM, the tensor and the special-function pipe are each busy 55 to 60 % of the time (2 x 4096
+// causal 56.5 and 56.5 %, ncu), under the power cap. What mattered (16 x 4096 causal, 32 / 8 heads x 128
+// unless said otherwise; here and below single kernels timed in short bursts: call after call, where the
+// power cap holds the clock down, the same shape takes 2120 to 2180 us for 1900 there):
 //   * the issuing warps stay converged and elect a lane, and every branch goes by a vote: descriptors
 //     are then uniform registers (from one lane in divergent code 4 x 4096 full: 1142 us, so 991);
 //   * one issuing warp per Q tile: a wait on a ready barrier costs such a warp some 200 cycles, and
-//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1904, with its registers 1874 to 1910;
-//     window 1024: 1304, 1097; 8 x 2048 causal, 16 heads x 64: 188, 137);
+//     with one warp for both the P of one tile waits behind the MMAs of the other (1978 us, so 1904,
+//     with its registers 1874 to 1910; window 1024: 1304, 1097; 8 x 2048 causal, 16 heads x 64: 188, 137);
 //   * cut tiles: one uniform test per visit, then bit masks (2900 -> 600 cycles for such a tile).
 // Measured and not taken: S shared by both tiles with P beside it (1016-1200 us on 4 x 4096 full
 // against 868-990), 64-key tiles with two S buffers each (1059; an MMA with N = 64 is bound by shared
 // memory, 48 cycles instead of 32), exponentials of the two tiles in forced turns (2064).
-// Every wait is bounded, see attention_common.cuh.
+// Every wait is bounded: 400 ms, counted from the CTA's last progress where it may last an item.
 #include "attention_common.cuh"
 #include "attention_issue.cuh"
 
@@ -155,6 +159,103 @@ __device__ __forceinline__ PlainItem plain_item(const AttnParams& p, int x, int 
   return w;
 }
 
+// Without the suspension of try_wait: whether the phase is complete now.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// mbar_wait for a whole converged warp, whose lanes all poll: every branch here goes by a vote, so
+// that the compiler knows that the warp stays together and keeps what follows in uniform registers.
+__device__ __forceinline__ bool mbar_poll_warp(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code) {
+  uint64_t t0 = 0;
+#pragma unroll 1
+  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 63u) == 63u) {
+      if (t0 == 0) t0 = global_ns();
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, global_ns() - t0 > ATT_WAIT_NS)) break;
+    }
+  }
+  *abort_flag = 1;
+  atomicOr(status, code);
+  return false;
+}
+static __device__ __noinline__ bool mbar_poll_warp_call(uint32_t bar, uint32_t parity,
+                                                        volatile int* abort_flag,
+                                                        unsigned int* status, unsigned code) {
+  return mbar_poll_warp(bar, parity, abort_flag, status, code);
+}
+// `INLINE` false: out of line but for the first poll (which the hardware suspends for a while), for
+// roles with few live registers: the code of a role that has to react fast stays small.
+template <bool INLINE>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code) {
+  if constexpr (INLINE) return mbar_poll_warp(bar, parity, abort_flag, status, code);
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __any_sync(0xffffffffu, mbar_poll_warp_call(bar, parity, abort_flag, status, code));
+}
+// A wait for something that takes as long as a whole work item (its row statistics, the next item): an
+// item may have any number of KV tiles, so the time counts from the last `progress` of the CTA.
+__device__ __forceinline__ bool mbar_poll_item(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code, volatile int* progress) {
+  uint64_t t0 = 0;
+  int seen = 0;
+#pragma unroll 1
+  for (uint32_t i = 0; i < ATT_WAIT_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 63u) == 63u) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      const int now = *progress;
+      if (__any_sync(0xffffffffu, t0 == 0 || now != seen)) {
+        seen = now;
+        t0 = global_ns();
+        i = 0;
+      } else if (__any_sync(0xffffffffu, global_ns() - t0 > ATT_WAIT_NS)) {
+        break;
+      }
+    }
+  }
+  *abort_flag = 1;
+  atomicOr(status, code);
+  return false;
+}
+static __device__ __noinline__ bool mbar_poll_item_call(uint32_t bar, uint32_t parity,
+                                                        volatile int* abort_flag,
+                                                        unsigned int* status, unsigned code,
+                                                        volatile int* progress) {
+  return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
+}
+template <bool INLINE>
+__device__ __forceinline__ bool mbar_wait_item(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* status,
+                                               unsigned code, volatile int* progress) {
+  if constexpr (INLINE) return mbar_poll_item(bar, parity, abort_flag, status, code, progress);
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __any_sync(0xffffffffu,
+                    mbar_poll_item_call(bar, parity, abort_flag, status, code, progress));
+}
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(is));
+  return is != 0;
+}
 // Cluster launch control: ask the hardware for the block index of a CTA of this grid that has not
 // been launched yet (it then never will be); the 16-byte answer arrives on an mbarrier.
 __device__ __forceinline__ void request_block(uint32_t dst, uint32_t bar) {
