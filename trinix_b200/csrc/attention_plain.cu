@@ -815,9 +815,11 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
       const bool foldable = BIAS == AP_GENERAL && sl2 > 0.0f && fabsf(kc) < 1e30f;
       // The row sum in four shares, one of every fourth pair of columns; in a tile each is a chain of
       // the 16 even and one of the 16 odd columns. The order of attention.cu, whose rows are held by
-      // four threads, so that the two agree to the last bit. Two chains and one share, 2 to 3 us in 200
-      // faster with ALiBi or a window (16 x 4096: 2288 / 2333 us, 4 x 3001 190.6 / 193.4; causal 2132 /
-      // 2119), leave a relative error of 1.4 / 2.0 x 2^-24 (rms, 4096 / 8192 keys), these 0.9 / 1.1.
+      // four threads, so that the two agree to the last bit. Two chains and one share leave a relative
+      // error of 1.4 / 2.0 x 2^-24 (rms, 4096 / 8192 keys), these 0.9 / 1.1, at the same speed within 1 to
+      // 3 % either way (16 x 4096 causal 2147 / 2131 us, with ALiBi 2294 / 2333, 4 x 3001 window 1024 191.2
+      // / 192.0, 2 x 2048 causal 74.0 / 76.6) as long as a pair is packed before it is added (else 2148,
+      // 2374, 193.7, 76.7).
       float m_run = -INFINITY;
       float2 l_run[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
       float m_ref = 0.0f;  // m_run, or 0 while no key has been visible
@@ -944,8 +946,8 @@ __global__ void __launch_bounds__(AP_THREADS, 1)
             const int c = 32 * g + 2 * i;
             const float2 x = fma2(pair_of(sr + c), unit2, neg2);
             const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-            sum[i & 3] = add2(sum[i & 3], e);
             pk[i] = pack16<BF16>(e.x, e.y);
+            sum[i & 3] = add2(sum[i & 3], e);
           }
           tmem_st16(s_addr + 16 * g, pk);
           if (g >= BN / 32 - 2) {
